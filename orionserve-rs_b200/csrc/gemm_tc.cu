@@ -204,6 +204,22 @@ __device__ __forceinline__ constexpr uint32_t instr_desc() {
          ((uint32_t)(M >> 4) << 24);
 }
 
+// Order in which the CTAs take the output tiles: eight token tiles against every weight tile before the next eight, token tiles first. In
+// blockIdx order a wave of 148 CTAs would meet nearly all weight tiles with one token tile, and a matrix larger than L2 would come from HBM
+// again for every 256 tokens; like this a wave works on about as many tokens as weight rows. UNIT: CTAs in x that stay together (a pair).
+struct TileXy {
+  uint32_t x, y;
+};
+constexpr uint32_t kRasterTokens = 8;
+template <uint32_t UNIT>
+__device__ __forceinline__ TileXy raster() {
+  if (gridDim.y == 1) return {blockIdx.x, 0};
+  const uint32_t units = gridDim.x / UNIT, id = blockIdx.y * units + blockIdx.x / UNIT;
+  const uint32_t first = id / (kRasterTokens * units) * kRasterTokens, in = id - first * units;
+  const uint32_t tall = min(kRasterTokens, gridDim.y - first);
+  return {in / tall * UNIT + blockIdx.x % UNIT, first + in % tall};
+}
+
 // ACT: the epilogue stores activations (kGemmGelu, kGemmRelu2, kGemmGeglu, kGemmStore); else f32 partials, or SwiGLU where `act` is given. A
 // template parameter, since the larger epilogue costs the weight-streaming shapes 0.8 us per launch.
 template <int TOKN, int WST, int XST, int MT, bool PAIR, bool ACT>
@@ -224,7 +240,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_ready + 1);
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t n0 = blockIdx.x * (MT * kTileN), t0 = blockIdx.y * TOKN, split = blockIdx.z;
+  const TileXy tile = raster<PAIR ? 2 : 1>();
+  const uint32_t n0 = tile.x * (MT * kTileN), t0 = tile.y * TOKN, split = blockIdx.z;
   const uint32_t nkb = (K + kSlabK - 1) / kSlabK;
   const uint32_t kb_begin = (uint32_t)((uint64_t)split * nkb / splits);
   const uint32_t kb_end = (uint32_t)((uint64_t)(split + 1) * nkb / splits);
