@@ -18,8 +18,8 @@
 //            token) and store f32 partials, 128 contiguous bytes per warp store.
 // Split-K: blockIdx.z owns a contiguous range of k slabs and writes its own slab
 // of the partial buffer; the consumer kernel sums the slabs.
-// Every CTA loads its own tiles, nothing is multicast. Clusters appear in two optional forms only: CTA pairs
-// for batches of 4096 rows and more (PAIR below), and the split-K reduction over distributed shared
+// Every CTA loads its own tiles, nothing is multicast. Clusters appear in two forms only: CTA pairs
+// for batches of more than 256 rows (gemm_pair_kernel), and the split-K reduction over distributed shared
 // memory (off by default). The activation producer can take its dependency from a counter in device
 // memory instead of the preceding kernel's completion (ReadyWait, used after a tensor-parallel hand-over).
 // Every wait is bounded; a wait that runs out sets a device error word and the
@@ -28,6 +28,7 @@
 
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -65,15 +66,10 @@ __device__ __forceinline__ void gtrace(uint32_t slot, int k) {
 // possible); prefill batches are tensor-bound and limited by the shared-memory fill rate, so a
 // CTA there takes two weight tiles against one activation tile (MT = 2: 64 KiB of operands per
 // 2.1 MFLOP instead of 48 KiB per 1.05), with two accumulators in tensor memory.
-// PAIR: two CTAs of a cluster work as one MMA unit (tcgen05 cta_group::2): each loads its own weight
-// tiles and HALF of the activation tile, the leader issues 256-row MMAs that read both CTAs' shared
-// memory and write both CTAs' tensor memory. Per CTA an activation stage is half as large, so a
-// prefill-sized projection moves 48 KiB of operands per 8.4 MFLOP instead of 64 KiB.
-template <int TOKN, int WST, int XST, int MT = 1, bool PAIR = false>
+template <int TOKN, int WST, int XST, int MT = 1>
 struct TcConfig {
   static constexpr int kWBytes = MT * kTileN * kSlabK * 2;
-  static constexpr int kXRows = PAIR ? TOKN / 2 : TOKN;  // activation rows this CTA loads per stage
-  static constexpr int kXBytes = kXRows * kSlabK * 2;
+  static constexpr int kXBytes = TOKN * kSlabK * 2;
   static constexpr int kWStages = WST;
   static constexpr int kXStages = XST;
   static constexpr int kXRingOffset = WST * kWBytes;
@@ -120,12 +116,6 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 }
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// Arrives on the barrier at cluster shared-memory address `bar_cluster_addr` (this CTA's or the
-// peer's) once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr)
-               : "memory");
 }
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                uint32_t accumulate) {
@@ -206,28 +196,24 @@ __device__ __forceinline__ constexpr uint32_t instr_desc() {
 
 // Order in which the CTAs take the output tiles: eight token tiles against every weight tile before the next eight, token tiles first. In
 // blockIdx order a wave of 148 CTAs would meet nearly all weight tiles with one token tile, and a matrix larger than L2 would come from HBM
-// again for every 256 tokens; like this a wave works on about as many tokens as weight rows. UNIT: CTAs in x that stay together (a pair).
+// again for every 256 tokens; like this a wave works on about as many tokens as weight rows.
 struct TileXy {
   uint32_t x, y;
 };
 constexpr uint32_t kRasterTokens = 8;
-template <uint32_t UNIT>
-__device__ __forceinline__ TileXy raster() {
-  if (gridDim.y == 1) return {blockIdx.x, 0};
-  const uint32_t units = gridDim.x / UNIT, id = blockIdx.y * units + blockIdx.x / UNIT;
-  const uint32_t first = id / (kRasterTokens * units) * kRasterTokens, in = id - first * units;
-  const uint32_t tall = min(kRasterTokens, gridDim.y - first);
-  return {in / tall * UNIT + blockIdx.x % UNIT, first + in % tall};
+__device__ __forceinline__ TileXy raster(uint32_t id, uint32_t tiles_x, uint32_t tiles_y) {
+  const uint32_t first = id / (kRasterTokens * tiles_x) * kRasterTokens, in = id - first * tiles_x, tall = min(kRasterTokens, tiles_y - first);
+  return {in / tall, first + in % tall};
 }
 
 // ACT: the epilogue stores activations (kGemmGelu, kGemmRelu2, kGemmGeglu, kGemmStore); else f32 partials, or SwiGLU where `act` is given. A
 // template parameter, since the larger epilogue costs the weight-streaming shapes 0.8 us per launch.
-template <int TOKN, int WST, int XST, int MT, bool PAIR, bool ACT>
+template <int TOKN, int WST, int XST, int MT, bool ACT>
 __global__ void __launch_bounds__(kThreads)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                float *__restrict__ partial, bf16 *__restrict__ act, uint32_t M, uint32_t N, uint32_t K,
                uint32_t splits, uint32_t cluster_reduce, uint32_t ldc, uint32_t epilogue, ReadyWait ready, const float *__restrict__ bias) {
-  using Cfg = TcConfig<TOKN, WST, XST, MT, PAIR>;
+  using Cfg = TcConfig<TOKN, WST, XST, MT>;
   extern __shared__ uint8_t raw_smem[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) &
                                               ~uintptr_t(1023));
@@ -240,15 +226,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_ready + 1);
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const TileXy tile = raster<PAIR ? 2 : 1>();
+  const TileXy tile = gridDim.y == 1 ? TileXy{blockIdx.x, 0} : raster(blockIdx.y * gridDim.x + blockIdx.x, gridDim.x, gridDim.y);
   const uint32_t n0 = tile.x * (MT * kTileN), t0 = tile.y * TOKN, split = blockIdx.z;
   const uint32_t nkb = (K + kSlabK - 1) / kSlabK;
   const uint32_t kb_begin = (uint32_t)((uint64_t)split * nkb / splits);
   const uint32_t kb_end = (uint32_t)((uint64_t)(split + 1) * nkb / splits);
   const uint32_t my_kb = kb_end - kb_begin;
-  // Pair mode: the two CTAs of a cluster sit next to each other in x; the even one leads.
-  const uint32_t pair_rank = PAIR ? (blockIdx.x & 1u) : 0u;
-  const bool leader = pair_rank == 0;
 
   pdl_trigger();
 #ifdef ORION_TRACE
@@ -276,20 +259,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     mbar_fence_init();
   }
   if (warp == 1) {
-    if (PAIR) {
-      tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);
-      tmem_relinquish_pair();
-    } else {
-      tmem_alloc(tmem_slot, Cfg::kTmemCols);
-      tmem_relinquish();
-    }
+    tmem_alloc(tmem_slot, Cfg::kTmemCols);
+    tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
-  if (PAIR) {  // the peer's barriers exist before anything of this CTA signals them
-    cluster_arrive_release();
-    cluster_wait_acquire();
-  }
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 #ifdef ORION_TRACE
@@ -305,16 +279,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       for (uint32_t i = 0; i < my_kb; ++i) {
         const uint32_t s = i % WST, use = i / WST;
         if (!mbar_wait(&empty_w[s], (use & 1) ^ 1)) { ok = false; break; }
-        if (PAIR) {
-          // both CTAs' tiles are counted on the leader's barrier, which expects the bytes of both
-          if (leader) mbar_arrive_expect_tx(&full_w[s], 2 * Cfg::kWBytes);
-          const uint32_t bar = mapa_u32(smem_u32(&full_w[s]), 0);
-#pragma unroll
-          for (int mt = 0; mt < MT; ++mt)
-            tma_load_2d_pair(w_ring + s * Cfg::kWBytes + mt * (kTileN * kSlabK * 2), &map_w, (int)((kb_begin + i) * kSlabK),
-                             (int)(n0 + mt * kTileN), bar);
-          continue;
-        }
         mbar_arrive_expect_tx(&full_w[s], Cfg::kWBytes);
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)  // rows past the matrix read as zeros and still count their bytes
@@ -335,19 +299,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       for (uint32_t i = 0; i < my_kb; ++i) {
         const uint32_t s = i % XST, use = i / XST;
         if (!mbar_wait(&empty_x[s], (use & 1) ^ 1)) { ok = false; break; }
-        if (PAIR) {  // this CTA's half of the token tile; counted on the leader's barrier like the weights
-          if (leader) mbar_arrive_expect_tx(&full_x[s], 2 * Cfg::kXBytes);
-          tma_load_2d_pair(x_ring + s * Cfg::kXBytes, &map_x, (int)((kb_begin + i) * kSlabK),
-                           (int)(t0 + pair_rank * Cfg::kXRows), mapa_u32(smem_u32(&full_x[s]), 0));
-          continue;
-        }
         mbar_arrive_expect_tx(&full_x[s], Cfg::kXBytes);
         tma_load_2d(x_ring + s * Cfg::kXBytes, &map_x, (int)((kb_begin + i) * kSlabK), (int)t0, &full_x[s]);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {  // in pair mode the leader issues for both CTAs
-      constexpr uint32_t idesc = PAIR ? instr_desc<TOKN, 2 * kTileN>() : instr_desc<TOKN>();
+    if (lane == 0) {
+      constexpr uint32_t idesc = instr_desc<TOKN>();
       for (uint32_t i = 0; i < my_kb; ++i) {
         const uint32_t sw = i % WST, sx = i % XST;
         if (!mbar_wait(&full_w[sw], (i / WST) & 1)) { ok = false; break; }
@@ -363,25 +321,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) {  // one accumulator of TOKN columns per weight tile
             const uint64_t a = smem_desc_sw128(wt + mt * (kTileN * kSlabK * 2) + k * kUmmaK * 2);
-            if (PAIR) umma_bf16_pair(tmem_base + (uint32_t)(mt * TOKN), a, b, idesc, (i > 0 || k > 0) ? 1u : 0u);
-            else umma_bf16(tmem_base + (uint32_t)(mt * TOKN), a, b, idesc, (i > 0 || k > 0) ? 1u : 0u);
+            umma_bf16(tmem_base + (uint32_t)(mt * TOKN), a, b, idesc, (i > 0 || k > 0) ? 1u : 0u);
           }
-        }
-        if (PAIR) {  // the same stage of both CTAs is free once these MMAs have read it
-#pragma unroll
-          for (uint32_t r = 0; r < 2; ++r) {
-            umma_commit_pair(mapa_u32(smem_u32(&empty_w[sw]), r));
-            umma_commit_pair(mapa_u32(smem_u32(&empty_x[sx]), r));
-          }
-          continue;
         }
         umma_commit(&empty_w[sw]);  // both stages are free once these MMAs have read them
         umma_commit(&empty_x[sx]);
       }
-      if (PAIR) {
-        umma_commit_pair(mapa_u32(smem_u32(acc_ready), 0));
-        umma_commit_pair(mapa_u32(smem_u32(acc_ready), 1));
-      } else
       umma_commit(acc_ready);  // arrives when every MMA above has completed
       ORION_GTRACE(tslot, 4);
     }
@@ -525,15 +470,241 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   if (!ok) atomicOr(&g_gemm_error, 1u);
   tc_fence_before();
   __syncthreads();
-  if (PAIR) {
-    // Neither CTA leaves, nor frees the tensor memory the pair allocated together, while the other may
-    // still be read by an MMA or be reading its accumulator.
-    cluster_arrive_release();
-    cluster_wait_acquire();
-    if (warp == 1) tmem_dealloc_pair(tmem_base, Cfg::kTmemCols);
-    return;
-  }
   if (warp == 1) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+}
+
+// ---- many rows: persistent CTA pairs ---------------------------------------------
+// Prompts and continuous batching (more than 256 rows) are bound by the tensor cores, with the rate at which operands reach shared memory close
+// behind. Two CTAs of a cluster work as one MMA unit (tcgen05 cta_group::2) on a tile of 256 weight rows x `tokn` tokens: each loads its own 128
+// weight rows and HALF of the token rows, so a k slab costs 32 KiB of loads per CTA for 4.2 MFLOP. The accumulator takes 256 of the 512 columns of
+// tensor memory; there are two, and the pairs stay on their SMs and go from tile to tile: the epilogue of one tile (the conversion of SwiGLU, 128 KiB
+// of f32 stores) runs under the main loop of the next, and the rings never drain in between. Tiles in the order of raster().
+struct PairConfig {
+  static constexpr int kMaxTokens = 256, kStages = 3, kStageK = 2 * kSlabK;
+  static constexpr int kWSlab = kTileN * kSlabK * 2, kXSlab = kMaxTokens / 2 * kSlabK * 2;  // 64 k of either operand
+  static constexpr int kWBytes = 2 * kWSlab, kXBytes = 2 * kXSlab;                          // one stage of either ring
+  static constexpr int kXRingOffset = kStages * kWBytes, kBarrierOffset = kXRingOffset + kStages * kXBytes;
+  static constexpr int kTmemCols = 512;
+  static constexpr int kSmemBytes = kBarrierOffset + 1024 /*align*/ + 512 /*barriers*/;
+  static constexpr uint32_t kEpilogueWarps = 4;
+};
+enum PairOutput : int { kPairPartials = 0, kPairSwiglu = 1, kPairAct = 2 };
+
+struct PairTile {
+  uint32_t n0, t0, split;
+};
+// Tile `id` of the launch: the k split slowest.
+__device__ __forceinline__ PairTile pair_tile_at(uint32_t id, uint32_t tiles_x, uint32_t tiles_y, uint32_t tokn) {
+  const uint32_t plane = tiles_x * tiles_y;
+  const TileXy t = raster(id % plane, tiles_x, tiles_y);
+  return {t.x * (2 * kTileN), t.y * tokn, id / plane};
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
+}
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// Arrives on this barrier in both CTAs of the pair once every MMA issued so far by this thread has completed.
+__device__ __forceinline__ void umma_commit_both(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3)
+               : "memory");
+}
+
+template <int OUT>
+__global__ void __launch_bounds__(kThreads)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, float *__restrict__ partial,
+                 bf16 *__restrict__ act, uint32_t M, uint32_t N, uint32_t K, uint32_t splits, uint32_t tokn, uint32_t ldc, uint32_t epilogue,
+                 ReadyWait ready, const float *__restrict__ bias) {
+  using Cfg = PairConfig;
+  constexpr uint32_t kStages = Cfg::kStages;
+  extern __shared__ uint8_t raw_smem[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
+  uint8_t *w_ring = smem, *x_ring = smem + Cfg::kXRingOffset;
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + Cfg::kBarrierOffset);
+  uint64_t *empty = full + kStages, *acc_full = empty + kStages, *acc_empty = acc_full + 2;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
+
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = blockIdx.x & 1u, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const bool leader = rank == 0;
+  const uint32_t nkb = (K + Cfg::kStageK - 1) / Cfg::kStageK;
+  const uint32_t tiles_x = (N + 2 * kTileN - 1) / (2 * kTileN), tiles_y = (M + tokn - 1) / tokn, total = tiles_x * tiles_y * splits;
+  auto slab_begin = [&](uint32_t split) { return (uint32_t)((uint64_t)split * nkb / splits); };
+
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    for (uint32_t s = 0; s < kStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 2 * Cfg::kEpilogueWarps);  // both CTAs' epilogues (used in the leader)
+    }
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_arrive_release();  // the peer's barriers exist before anything of this CTA signals them
+  cluster_wait_acquire();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  bool ok = true;
+
+  if (warp == 0) {
+    // Producer: this CTA's weight rows and its half of the token rows; the bytes of both CTAs are counted on the leader's barrier. Weights are
+    // immutable: those of the first slabs are asked for before the wait for the kernel that makes the activations.
+    // The whole warp runs the loop and one elected lane issues, here and below: addresses and descriptors stay in uniform registers.
+    const uint32_t half = tokn / 2, x_bytes = 2 * half * kSlabK * 2;
+    const bool elected = elect_one();
+    uint32_t it = 0, early = 0;
+    auto load_w = [&](uint32_t s, uint32_t kb, uint32_t n0) {
+      if (!elected) return;
+      const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
+      if (leader) mbar_arrive_expect_tx(&full[s], 2 * (Cfg::kWBytes + x_bytes));
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        tma_load_2d_pair(w_ring + s * Cfg::kWBytes + j * Cfg::kWSlab, &map_w, (int)(kb * Cfg::kStageK + j * kSlabK), (int)(n0 + rank * kTileN), bar);
+    };
+    {
+      const PairTile tile = pair_tile_at(pair, tiles_x, tiles_y, tokn);
+      for (uint32_t kb = slab_begin(tile.split), end = slab_begin(tile.split + 1); kb < end && early < kStages; ++kb, ++early) load_w(early, kb, tile.n0);
+    }
+    if (ready.counter) {
+      if (!wait_ready(ready)) atomicOr(&g_gemm_error, 2u);
+      fence_proxy_async_all();
+    } else {
+      pdl_wait();
+    }
+    for (uint32_t t = pair; ok && t < total; t += pairs) {
+      const PairTile tile = pair_tile_at(t, tiles_x, tiles_y, tokn);
+      for (uint32_t kb = slab_begin(tile.split), end = slab_begin(tile.split + 1); kb < end; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        if (it >= early) {
+          if (!mbar_wait(&empty[s], ((it / kStages) & 1) ^ 1)) { ok = false; break; }
+          load_w(s, kb, tile.n0);
+        }
+        if (elected) {
+          const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            tma_load_2d_pair(x_ring + s * Cfg::kXBytes + j * Cfg::kXSlab, &map_x, (int)(kb * Cfg::kStageK + j * kSlabK), (int)(tile.t0 + rank * half), bar);
+        }
+        __syncwarp();
+      }
+    }
+    // the slots that are still being read: nobody signals a barrier of a CTA that is gone
+    for (uint32_t i = it > kStages ? it - kStages : 0; ok && i < it; ++i) ok = mbar_wait(&empty[i % kStages], (i / kStages) & 1);
+  } else if (warp == 1) {
+    if (leader) {  // the leader issues for both CTAs
+      const uint32_t idesc = instr_desc<0, 2 * kTileN>() | ((tokn >> 3) << 17);
+      const uint64_t w_desc = smem_desc_sw128(smem_u32(w_ring)), x_desc = smem_desc_sw128(smem_u32(x_ring));
+      const bool elected = elect_one();
+      uint32_t it = 0, turn = 0;
+      for (uint32_t t = pair; ok && t < total; t += pairs, ++turn) {
+        const PairTile tile = pair_tile_at(t, tiles_x, tiles_y, tokn);
+        const uint32_t buf = turn & 1, acc = tmem_base + buf * Cfg::kMaxTokens;
+        if (!mbar_wait(&acc_empty[buf], ((turn >> 1) & 1) ^ 1)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t begin = slab_begin(tile.split), end = slab_begin(tile.split + 1);
+        for (uint32_t kb = begin; kb < end; ++kb, ++it) {
+          const uint32_t s = it % kStages;
+          if (!mbar_wait(&full[s], (it / kStages) & 1)) { ok = false; break; }
+          tc_fence_after();
+          if (elected) {
+            const uint64_t a = w_desc + s * (Cfg::kWBytes >> 4), b = x_desc + s * (Cfg::kXBytes >> 4);
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int k = 0; k < kSlabK / kUmmaK; ++k)  // 16 k elements inside the swizzle atom = 32 bytes on the start address
+                umma_bf16_pair(acc, a + (j * Cfg::kWSlab + k * kUmmaK * 2 >> 4), b + (j * Cfg::kXSlab + k * kUmmaK * 2 >> 4), idesc,
+                               (kb > begin || j > 0 || k > 0) ? 1u : 0u);
+            umma_commit_both(&empty[s]);  // the stage of both CTAs is free once these MMAs have read it
+          }
+          __syncwarp();
+        }
+        if (ok && elected) umma_commit_both(&acc_full[buf]);
+      }
+    }
+  } else if (warp >= 4) {
+    // Epilogue: warp w reads tensor-memory lanes 32 * (w % 4) .. + 31 (lane = weight row, column = token).
+    const uint32_t lq = warp & 3;
+    // The output may still be read by the kernel before the producer of x. (With a ready counter the producer has read it before it counted.)
+    if (!ready.counter) pdl_wait();
+    constexpr uint32_t kBatch = 4;  // 16-column loads in flight before one wait
+    uint32_t turn = 0;
+    for (uint32_t t = pair; ok && t < total; t += pairs, ++turn) {
+      const PairTile tile = pair_tile_at(t, tiles_x, tiles_y, tokn);
+      const uint32_t buf = turn & 1, acc = tmem_base + ((lq * 32u) << 16) + buf * Cfg::kMaxTokens;
+      const uint32_t n = tile.n0 + rank * kTileN + lq * 32 + lane, t0 = tile.t0;
+      if (!mbar_wait(&acc_full[buf], (turn >> 1) & 1)) { ok = false; break; }
+      tc_fence_after();
+      float *dst = partial + (size_t)tile.split * M * N;
+      const float b_n = OUT == kPairAct && bias && n < N ? bias[n] : 0.f;
+#pragma unroll 1
+      for (uint32_t mb = 0; mb < tokn; mb += 16 * kBatch) {
+        uint32_t rr[kBatch][16];
+#pragma unroll
+        for (uint32_t b = 0; b < kBatch; ++b)
+          if (mb + 16 * b < tokn) tmem_ld16(acc + mb + 16 * b, rr[b]);
+        tmem_ld_wait();
+        if (mb + 16 * kBatch >= tokn) {  // the last of this accumulator is in registers: the MMAs of the tile after the next may write it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[buf]), 0));
+        }
+#pragma unroll
+        for (uint32_t b = 0; b < kBatch; ++b) {
+          const uint32_t c = mb + 16 * b;
+          if (c >= tokn || t0 + c >= M) continue;  // warp-uniform
+          uint32_t (&r)[16] = rr[b];
+          if (OUT == kPairPartials) {
+            if (n < N) {
+#pragma unroll
+              for (uint32_t j = 0; j < 16; ++j)
+                if (t0 + c + j < M) dst[(size_t)(t0 + c + j) * ldc + n] = __uint_as_float(r[j]);
+            }
+          } else if (OUT == kPairSwiglu || epilogue == kGemmGeglu) {
+            // Weight rows are interleaved: lane 2i holds gate f, lane 2i + 1 up f of these 16 tokens. The lanes of a pair trade halves and each
+            // finishes one token of every two (SwiGLU: tensor.rs:167-189).
+            const uint32_t odd = lane & 1u, stride = OUT == kPairSwiglu ? N >> 1 : ldc;
+            bf16 *out = act + (size_t)(t0 + c) * stride + (n >> 1);
+#pragma unroll
+            for (uint32_t jj = 0; jj < 8; ++jj) {
+              const uint32_t recv = __shfl_xor_sync(0xffffffffu, odd ? r[2 * jj] : r[2 * jj + 1], 1), j = 2 * jj + odd;
+              const float g = __uint_as_float(odd ? recv : r[2 * jj]), u = __uint_as_float(odd ? r[2 * jj + 1] : recv);
+              const float v = OUT == kPairSwiglu ? __fmul_rn(g / (1.0f + __expf(-g)), u) : gelu_tanh<bf16>(g) * u;
+              if (t0 + c + j < M && n < N) out[(size_t)j * stride] = __float2bfloat16_rn(v);
+            }
+          } else if (n < N) {
+            bf16 *out = act + (size_t)(t0 + c) * ldc + n;
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) {
+              const float v = __uint_as_float(r[j]) + b_n;
+              if (t0 + c + j < M) out[(size_t)j * ldc] = __float2bfloat16_rn(epilogue == kGemmGelu ? gelu_tanh<bf16>(v) : (epilogue == kGemmRelu2 ? relu2(v) : v));
+            }
+          }
+        }
+      }
+    }
+  }
+  if (!ok) atomicOr(&g_gemm_error, 1u);
+  tc_fence_before();
+  __syncthreads();
+  // Neither CTA leaves, nor frees the tensor memory the pair allocated together, while the other may still be read by an MMA or be reading
+  // its accumulator.
+  cluster_arrive_release();
+  cluster_wait_acquire();
+  if (warp == 1) tmem_dealloc_pair(tmem_base, Cfg::kTmemCols);
 }
 
 // ---- host side -----------------------------------------------------------------
@@ -600,55 +771,108 @@ int cached_map(const void *base, uint64_t rows, uint64_t k, uint64_t ld, uint32_
   return ORION_OK;
 }
 
-template <bool ACT, int TOKN, int WST, int XST, int MT, bool PAIR>
+template <bool ACT, int TOKN, int WST, int XST, int MT>
 int launch_tc_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float *partial, bf16 *act,
               uint32_t rows, uint32_t n, uint32_t k, uint32_t splits, bool cluster_reduce, uint32_t ldc, GemmEpilogue epi,
               cudaStream_t stream, ReadyWait ready, const float *bias) {
   if (ldc == 0) ldc = n;
   if (ldc != n && (splits != 1 || epi == kGemmSwiglu))
     return set_error(ORION_ERR_INTERNAL, "a strided GEMM output needs one k split and no SwiGLU");
-  using Cfg = TcConfig<TOKN, WST, XST, MT, PAIR>;
+  using Cfg = TcConfig<TOKN, WST, XST, MT>;
   static_assert(Cfg::kSmemBytes <= 232448, "ring exceeds the shared memory of an SM");
   if (MT > 1 && cluster_reduce) return set_error(ORION_ERR_INTERNAL, "cluster split-K is built for one weight tile per CTA");
   static bool attr_set[kMaxDeviceOrdinals] = {};
-  ORION_CUDA_CHECK("gemm_tc attr", ensure_dynamic_smem(gemm_tc_kernel<TOKN, WST, XST, MT, PAIR, ACT>, Cfg::kSmemBytes, attr_set));
+  ORION_CUDA_CHECK("gemm_tc attr", ensure_dynamic_smem(gemm_tc_kernel<TOKN, WST, XST, MT, ACT>, Cfg::kSmemBytes, attr_set));
   const CUtensorMap *mw, *mx;
   ORION_TRY(cached_map(w, n, k, ldw, kTileN, &mw));
-  ORION_TRY(cached_map(x, rows, k, ldx, Cfg::kXRows, &mx));
+  ORION_TRY(cached_map(x, rows, k, ldx, TOKN, &mx));
   dim3 grid((n + MT * kTileN - 1) / (MT * kTileN), (rows + TOKN - 1) / TOKN, splits);
-  if (PAIR) {
-    if (cluster_reduce || (grid.x & 1u))
-      return set_error(ORION_ERR_INTERNAL, "the paired GEMM needs an even number of weight tile groups and no cluster split-K");
-    ORION_CUDA_CHECK("gemm_tc", launch_pdl_cluster(gemm_tc_kernel<TOKN, WST, XST, MT, PAIR, ACT>, grid, dim3(kThreads), dim3(2, 1, 1),
-                                                   Cfg::kSmemBytes, stream, *mw, *mx, partial, act, rows, n, k, splits,
-                                                   0u, ldc, (uint32_t)epi, ready, bias));
-  } else if (cluster_reduce)
-    ORION_CUDA_CHECK("gemm_tc", launch_pdl_cluster(gemm_tc_kernel<TOKN, WST, XST, MT, PAIR, ACT>, grid, dim3(kThreads), dim3(1, 1, splits),
+  if (cluster_reduce)
+    ORION_CUDA_CHECK("gemm_tc", launch_pdl_cluster(gemm_tc_kernel<TOKN, WST, XST, MT, ACT>, grid, dim3(kThreads), dim3(1, 1, splits),
                                                    Cfg::kSmemBytes, stream, *mw, *mx, partial, act, rows, n, k, splits,
                                                    1u, ldc, (uint32_t)epi, ready, bias));
   else
-    ORION_CUDA_CHECK("gemm_tc", launch_pdl(gemm_tc_kernel<TOKN, WST, XST, MT, PAIR, ACT>, grid, dim3(kThreads), Cfg::kSmemBytes, stream,
+    ORION_CUDA_CHECK("gemm_tc", launch_pdl(gemm_tc_kernel<TOKN, WST, XST, MT, ACT>, grid, dim3(kThreads), Cfg::kSmemBytes, stream,
                                            *mw, *mx, partial, act, rows, n, k, splits, 0u, ldc, (uint32_t)epi, ready, bias));
   count_launch();
   ORION_CUDA_CHECK("gemm_tc", cudaGetLastError());
   return ORION_OK;
 }
 
-template <int TOKN, int WST, int XST, int MT = 1, bool PAIR = false>
+template <int TOKN, int WST, int XST, int MT = 1>
 int launch_tc(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float *partial, bf16 *act, uint32_t rows, uint32_t n,
               uint32_t k, uint32_t splits, bool cluster_reduce, uint32_t ldc, GemmEpilogue epi, cudaStream_t stream, ReadyWait ready,
               const float *bias) {
-  auto form = epi == kGemmGelu || epi == kGemmStore || epi == kGemmRelu2 || epi == kGemmGeglu ? launch_tc_form<true, TOKN, WST, XST, MT, PAIR>
-                                                    : launch_tc_form<false, TOKN, WST, XST, MT, PAIR>;
+  auto form = epi == kGemmGelu || epi == kGemmStore || epi == kGemmRelu2 || epi == kGemmGeglu ? launch_tc_form<true, TOKN, WST, XST, MT>
+                                                    : launch_tc_form<false, TOKN, WST, XST, MT>;
   return form(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias);
 }
 
-// 256-token tiles as CTA pairs (tcgen05 cta_group::2). Measured on the Llama-3-8B shape, projections of
-// a step of 512 / 2048 / 8192 tokens: 616 / 869 / 1034 TFLOP/s paired against 630 / 900 / 996 unpaired:
-// the pair pays off once a step has many token tiles. 1 (default) = pairs from 4096 rows on, 2 = wherever
-// the grid allows (the parity tests run this), 0 = never. ORION_GEMM_PAIR overrides.
+// How a projection of many rows is cut for the persistent pairs: 74 pairs take the tiles (and k splits) round by round, so the time is the number of
+// rounds times a tile's. Unit: 1.14 ns, what one token column costs a k slab of 64. A slab takes the tensor cores tokn + 16 units (measured 311 ns
+// with 256 tokens, 162 with 128, few tiles at work), and with all pairs at work the loads of 256 + tokn rows, which reach shared memory at 14 TB/s in
+// all (359-399 ns with 256 tokens, 285-308 with 192, 240-255 with 128). About 3 us for the last tile's epilogue; the consumer reads every k split's
+// slab again. Against a sweep of 22 shapes of 300 to 7006 rows, every tile and 1 to 4 splits, the choice is 1.8 % off the best on average.
+constexpr uint32_t kPairs = 74;
+uint32_t pair_tiles(uint32_t rows, uint32_t n, uint32_t tokn) { return (n + 2 * kTileN - 1) / (2 * kTileN) * ((rows + tokn - 1) / tokn); }
+uint64_t pair_cost(uint32_t rows, uint32_t n, uint32_t k, uint32_t splits, uint32_t tokn) {
+  const uint64_t stages = (k + PairConfig::kStageK - 1) / PairConfig::kStageK, slabs = 2 * ((stages + splits - 1) / splits);
+  const uint64_t tiles = (uint64_t)pair_tiles(rows, n, tokn) * splits, rounds = (tiles + kPairs - 1) / kPairs;
+  const uint64_t slab = std::max<uint64_t>(tokn + 16, std::min<uint64_t>(tiles, kPairs) * (2 * kTileN + tokn) / 128);
+  return rounds * (slabs * slab + 2 * tokn) + 9 * tokn + (uint64_t)(splits - 1) * ((rows + 15) / 16 * 16) * n / 1300;
+}
+uint32_t pair_tokens(uint32_t rows, uint32_t n, uint32_t k, uint32_t splits) {
+  uint32_t best = PairConfig::kMaxTokens;
+  for (uint32_t t = best - 16; t >= 128; t -= 16)
+    if (pair_cost(rows, n, k, splits, t) < pair_cost(rows, n, k, splits, best)) best = t;
+  return best;
+}
+// A k split has to gain a tenth: it keeps an activation out of the epilogue. Two full rounds and more are never split. The same for all row counts
+// of a run 16 j + 1 .. 16 (j + 1), since token tiles are multiples of 16.
+uint32_t pair_splits(uint32_t rows, uint32_t n, uint32_t k) {
+  uint32_t best = 1;
+  if (pair_tiles(rows, n, PairConfig::kMaxTokens) > 2 * kPairs) return best;
+  uint64_t cost = pair_cost(rows, n, k, 1, pair_tokens(rows, n, k, 1)) * 9 / 10;
+  for (uint32_t s = 2; s <= 4 && k / s >= 8 * kSlabK; ++s) {
+    const uint64_t c = pair_cost(rows, n, k, s, pair_tokens(rows, n, k, s));
+    if (c < cost) best = s, cost = c;
+  }
+  return best;
+}
+
+template <int OUT>
+int launch_pair_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float *partial, bf16 *act, uint32_t rows, uint32_t n, uint32_t k,
+                     uint32_t splits, uint32_t ldc, GemmEpilogue epi, cudaStream_t stream, ReadyWait ready, const float *bias) {
+  if (ldc == 0) ldc = n;
+  if (ldc != n && (splits != 1 || epi == kGemmSwiglu))
+    return set_error(ORION_ERR_INTERNAL, "a strided GEMM output needs one k split and no SwiGLU");
+  using Cfg = PairConfig;
+  static_assert(Cfg::kSmemBytes <= 232448, "ring exceeds the shared memory of an SM");
+  static bool attr_set[kMaxDeviceOrdinals] = {};
+  ORION_CUDA_CHECK("gemm_pair attr", ensure_dynamic_smem(gemm_pair_kernel<OUT>, Cfg::kSmemBytes, attr_set));
+  const uint32_t tokn = pair_tokens(rows, n, k, splits);
+  const CUtensorMap *mw, *mx;
+  ORION_TRY(cached_map(w, n, k, ldw, kTileN, &mw));
+  ORION_TRY(cached_map(x, rows, k, ldx, tokn / 2, &mx));
+  const uint32_t tiles = pair_tiles(rows, n, tokn) * splits;
+  ORION_CUDA_CHECK("gemm_pair", launch_pdl_cluster(gemm_pair_kernel<OUT>, dim3(2 * std::min(tiles, kPairs)), dim3(kThreads), dim3(2, 1, 1), Cfg::kSmemBytes,
+                                                   stream, *mw, *mx, partial, act, rows, n, k, splits, tokn, ldc, (uint32_t)epi, ready, bias));
+  count_launch();
+  ORION_CUDA_CHECK("gemm_pair", cudaGetLastError());
+  return ORION_OK;
+}
+
+int launch_pair(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float *partial, bf16 *act, uint32_t rows, uint32_t n, uint32_t k,
+                uint32_t splits, uint32_t ldc, GemmEpilogue epi, cudaStream_t stream, ReadyWait ready, const float *bias) {
+  auto form = epi == kGemmPartials ? launch_pair_form<kPairPartials> : (epi == kGemmSwiglu ? launch_pair_form<kPairSwiglu> : launch_pair_form<kPairAct>);
+  return form(x, ldx, w, ldw, partial, act, rows, n, k, splits, ldc, epi, stream, ready, bias);
+}
+
+// Who takes the persistent pairs: 1 (default) = batches of more than 256 rows, 2 = of more than 128 (the parity tests run this), 0 = nobody.
+// ORION_GEMM_PAIR overrides. The four projections of the 8B shape at 512 / 2048 / 8192 rows, f32 out: 188 / 611 / 2380 us with pairs, 239 / 775 / 2540
+// with one CTA per 256-token tile. At 129 to 256 rows the two are equal: the wider gate/up 3-6 % slower with pairs, the others 5-13 % faster.
 int g_gemm_pair = std::getenv("ORION_GEMM_PAIR") ? std::atoi(std::getenv("ORION_GEMM_PAIR")) : 1;
-constexpr uint32_t kPairMinRows = 4096;
+bool takes_pairs(uint32_t rows) { return g_gemm_pair >= 1 && rows > (g_gemm_pair >= 2 ? 128u : 256u); }
 
 // Tuning A/B: ORION_GEMM_PREFILL_TILES=1 keeps one weight tile per CTA for prefill-sized batches
 // (two tiles measured 3 % faster on the continuous-batching workload, gate/up only: the other
@@ -710,6 +934,10 @@ int launch_gemm_tc(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, flo
   uint32_t tt = token_tile(rows);
   // prefill batches whose 256-token tiles would leave SMs idle take 128-token tiles instead
   if (rows > 256 && g_prefill_fill == 1 && ((n + kTileN - 1) / kTileN) * ((rows + 255) / 256) < 148) tt = 128;
+  if (takes_pairs(rows) && !cluster_reduce) {
+    if (splits > (k + PairConfig::kStageK - 1) / PairConfig::kStageK) return set_error(ORION_ERR_INTERNAL, "gemm split count %u leaves a split empty", splits);
+    return launch_pair(x, ldx, w, ldw, partial, act, rows, n, k, splits, ldc, epi, stream, ready, bias);
+  }
   switch (tt) {
     case 16:
       return deep ? launch_tc<16, 6, 3>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias)
@@ -726,14 +954,8 @@ int launch_gemm_tc(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, flo
                  : launch_tc<128, 6, 6>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias);
     default: {
       const uint32_t mt = (!cluster_reduce && prefill_weight_tiles(rows, n) == 2) ? 2 : 1;
-      // CTA pairs: each CTA loads half of the activation tile, so the rings go a stage deeper
-      const bool pair = (g_gemm_pair >= 2 || (g_gemm_pair == 1 && rows >= kPairMinRows)) && !cluster_reduce &&
-                        (((n + mt * kTileN - 1) / (mt * kTileN)) & 1u) == 0;
-      if (mt == 2)
-        return pair ? launch_tc<256, 4, 4, 2, true>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias)
-                    : launch_tc<256, 3, 3, 2>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias);
-      return pair ? launch_tc<256, 6, 6, 1, true>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias)
-                  : launch_tc<256, 4, 4>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias);
+      return mt == 2 ? launch_tc<256, 3, 3, 2>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias)
+                     : launch_tc<256, 4, 4>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias);
     }
   }
 }
@@ -796,6 +1018,10 @@ GemmPlan gemm_plan(bool is_bf16, uint32_t rows, uint32_t n, uint32_t k, uint32_t
         encode_fn() != nullptr))
     return p;
   p.tensor_core = true;
+  if (takes_pairs(rows)) {
+    p.splits = p.out_slabs = pair_splits(rows, n, k);
+    return p;
+  }
   if (rows > 256) {
     // Prefill-sized batches are tensor-bound; the 256-token tiles take a whole SM each (192 KiB of
     // rings), so a projection with few weight tiles (N = 4096: 32) needs k splits to reach all SMs.
@@ -831,7 +1057,7 @@ GemmPlan gemm_plan(bool is_bf16, uint32_t rows, uint32_t n, uint32_t k, uint32_t
 size_t gemm_partial_floats(bool is_bf16, uint32_t max_rows, uint32_t n, uint32_t k) {
   size_t best = (size_t)max_rows * n;
   if (!is_bf16) return best;
-  for (uint32_t r = 1; r <= max_rows; ++r) {
+  for (uint32_t r = 1; r <= max_rows; r = takes_pairs(r) && r < max_rows ? std::min(max_rows, (r / 16 + 1) * 16) : r + 1) {  // as in pair_splits
     const GemmPlan p = gemm_plan(true, r, n, k, k, k);
     const size_t need = (size_t)p.splits * r * n;
     if (need > best) best = need;
