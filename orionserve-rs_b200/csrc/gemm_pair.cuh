@@ -8,7 +8,10 @@
 // the warp and one elected lane issues, stages hold 128 k, and ONE commit a stage frees both CTAs' halves. Measured on 8192 x 14336 x 4096: one lane
 // in a divergent branch with four commits every 64 k 735 us, with one commit 617, like this 612; with 128 tokens a tile 1310, 994, 799.
 //
-// A CTA has 256 threads: warp 0 loads, warp 1 of the leader issues the MMAs, warps 4-7 are the epilogue. Every wait is bounded; a wait that runs out
+// The epilogue has eight warps: with four, the activations of a mixture (k 2048, 13 us of main loop a tile) took longer than the main loop (up
+// projection of 7006 rows, 331 us against 210; of 2048 rows with the exact GELU, 125 against 87).
+//
+// A CTA has 384 threads: warp 0 loads, warp 1 of the leader issues the MMAs, warps 4-11 are the epilogue. Every wait is bounded; a wait that runs out
 // sets the error word, and the CTAs still free their tensor memory.
 #pragma once
 
@@ -81,12 +84,12 @@ __device__ __forceinline__ TileXy raster(uint32_t id, uint32_t tiles_x, uint32_t
 }
 
 struct PairConfig {
-  static constexpr uint32_t kThreads = 256, kRows = 128, kSlabK = 64;  // threads and weight rows per CTA, k of a TMA box (one swizzle atom)
+  static constexpr uint32_t kThreads = 384, kRows = 128, kSlabK = 64;  // threads and weight rows per CTA, k of a TMA box (one swizzle atom)
   static constexpr uint32_t kMaxTokens = 256, kStages = 3, kStageK = 2 * kSlabK;
   static constexpr uint32_t kWSlab = kRows * kSlabK * 2, kXSlab = kMaxTokens / 2 * kSlabK * 2;  // 64 k of either operand
   static constexpr uint32_t kWBytes = 2 * kWSlab, kXBytes = 2 * kXSlab;                          // one stage of either ring
   static constexpr uint32_t kXRingOffset = kStages * kWBytes, kBarrierOffset = kXRingOffset + kStages * kXBytes;
-  static constexpr uint32_t kTmemCols = 512, kEpilogueWarps = 4;
+  static constexpr uint32_t kTmemCols = 512, kEpilogueWarps = 8;
   static constexpr int kSmemBytes = kBarrierOffset + 1024 /*align*/ + 512 /*barriers*/;
   static_assert(kSmemBytes <= 232448, "ring exceeds the shared memory of an SM");
 };
@@ -101,9 +104,10 @@ struct PairJob {
 // The body of a kernel of pairs (grid: two CTAs each, cluster of two). Work provides
 //   total()          tiles of the launch
 //   early(id)        whether tile `id` is known before the preceding kernel has ended
-//   job(id)          the tile; one without stages (kb == end) is passed over
+//   job(id)          the tile, a Job; one without stages (kb == end) is passed over
 //   x_box()          token rows of a box of every x map: at least half of any tile's columns, a multiple of 8
-//   store(id, c, r)  a warp's 16 columns c .. c + 15 of its 32 weight rows, f32
+//   Job              what job() returns: a PairJob, and what store() needs
+//   store(j, row, c, r)  columns c .. c + 15 of weight row w_row + row (of 32 in a warp, one a lane), f32
 template <typename Work>
 __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uint32_t *error) {
   using Cfg = PairConfig;
@@ -160,7 +164,7 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
         tma_load_2d_pair(w_ring + s * Cfg::kWBytes + h * Cfg::kWSlab, j.w, (int)(kb * Cfg::kStageK + h * Cfg::kSlabK), (int)(j.w_row + rank * Cfg::kRows), bar);
     };
     if (pair < total && work.early(pair)) {
-      const PairJob j = work.job(pair);
+      const typename Work::Job j = work.job(pair);
       for (uint32_t kb = j.kb; kb < j.end && early < kStages; ++kb, ++early) load_w(early, kb, j);
     }
     if (ready.counter) {
@@ -170,7 +174,7 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
       pdl_wait();
     }
     for (uint32_t t = pair; ok && t < total; t += pairs) {
-      const PairJob j = work.job(t);
+      const typename Work::Job j = work.job(t);
       for (uint32_t kb = j.kb; kb < j.end; ++kb, ++it) {
         const uint32_t s = it % kStages;
         if (it >= early) {
@@ -195,7 +199,7 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
       if (!Work::kStaticTiles) pdl_wait();  // the list of tiles
       uint32_t it = 0, turn = 0;
       for (uint32_t t = pair; ok && t < total; t += pairs) {
-        const PairJob j = work.job(t);
+        const typename Work::Job j = work.job(t);
         if (j.kb >= j.end) continue;
         const uint32_t id = idesc(2 * Cfg::kRows, j.cols, false), buf = turn & 1, acc = tmem_base + buf * Cfg::kMaxTokens;
         if (!mbar_wait(&acc_empty[buf], ((turn >> 1) & 1) ^ 1)) { ok = false; break; }
@@ -220,33 +224,39 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
       }
     }
   } else if (warp >= 4) {
-    // Epilogue: warp w reads tensor-memory lanes 32 * (w % 4) .. + 31 (lane = weight row, column = token).
+    // Epilogue: warp w reads tensor-memory lanes 32 * (w % 4) .. + 31 (lane = weight row, column = token); the two warps of the same lanes take
+    // turns, a batch of columns each.
     // The output may still be read by the kernel before the producer of x. (With a ready counter the producer has read it before it counted.)
     if (!ready.counter) pdl_wait();
     constexpr uint32_t kBatch = Work::kBatch;  // 16-column loads in flight before one wait
     uint32_t turn = 0;
     for (uint32_t t = pair; ok && t < total; t += pairs) {
-      const PairJob j = work.job(t);
+      const typename Work::Job j = work.job(t);
       if (j.kb >= j.end) continue;
       const uint32_t buf = turn & 1, acc = tmem_base + (((warp & 3) * 32u) << 16) + buf * Cfg::kMaxTokens;
       if (!mbar_wait(&acc_full[buf], (turn >> 1) & 1)) { ok = false; break; }
       ++turn;
       tc_fence_after();
+      constexpr uint32_t kStep = 16 * kBatch * (Cfg::kEpilogueWarps / 4);
+      uint32_t mb = 16 * kBatch * ((warp - 4) / 4);
+      // once this warp's last columns are in registers, the MMAs of the tile after the next may write them
+      auto release = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[buf]), 0));
+      };
+      if (mb >= j.cols) release();
 #pragma unroll 1
-      for (uint32_t mb = 0; mb < j.cols; mb += 16 * kBatch) {
+      for (; mb < j.cols; mb += kStep) {
         uint32_t rr[kBatch][16];
 #pragma unroll
         for (uint32_t b = 0; b < kBatch; ++b)
           if (mb + 16 * b < j.cols) tmem_ld16(acc + mb + 16 * b, rr[b]);
         tmem_ld_wait();
-        if (mb + 16 * kBatch >= j.cols) {  // the last of this accumulator is in registers: the MMAs of the tile after the next may write it
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[buf]), 0));
-        }
+        if (mb + kStep >= j.cols) release();
 #pragma unroll
         for (uint32_t b = 0; b < kBatch; ++b)
-          if (mb + 16 * b < j.cols) work.store(t, j, rank * Cfg::kRows + (warp & 3) * 32 + lane, mb + 16 * b, rr[b]);
+          if (mb + 16 * b < j.cols) work.store(j, rank * Cfg::kRows + (warp & 3) * 32 + lane, mb + 16 * b, rr[b]);
       }
     }
   }

@@ -24,9 +24,7 @@
 // memory instead of the preceding kernel's completion (ReadyWait, used after a tensor-parallel hand-over).
 // Every wait is bounded; a wait that runs out sets a device error word and the
 // CTA still releases its tensor memory before returning.
-#include "kernels.h"
-
-#include <cuda.h>
+#include "gemm_pair.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -79,133 +77,11 @@ struct TcConfig {
   static constexpr int kSmemBytes = kBarrierOffset + 1024 /*align*/ + 512 /*barriers*/;
 };
 
-__device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                   smem_u32(dst_smem)),
-               "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// ---- cta_group::2 (a pair of CTAs as one MMA unit) ----
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t *dst_smem, uint32_t ncols) {  // one warp in EACH CTA of the pair
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// 2-D tiled TMA load of one CTA of a pair: the data lands in THIS CTA's shared memory, the bytes are
-// counted on the barrier at cluster address `bar_cluster_addr` (the leader's). No multicast.
-__device__ __forceinline__ void tma_load_2d_pair(void *dst_smem, const void *tensor_map, int c0, int c1,
-                                                 uint32_t bar_cluster_addr) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst_smem)),
-      "l"(tensor_map), "r"(c0), "r"(c1), "r"(bar_cluster_addr)
-      : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void cluster_arrive_release() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait_acquire() {
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Address of the same shared-memory location in cluster member `rank`.
-__device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
-__device__ __forceinline__ void tmem_ld_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major tile stored as rows of 128 bytes
-// with the 128-byte swizzle: 8-row groups are 1024 bytes apart (stride offset),
-// the leading offset is unused for swizzled K-major tiles (encoded 1),
-// descriptor version 1, layout type 2 (128-byte swizzle).
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
-// Instruction descriptor: f32 accumulate, bf16 x bf16, both operands K-major,
-// N = TOKN (>>3 at bit 17), M = 128 (>>4 at bit 24).
-template <int TOKN, int M = kTileN>
-__device__ __forceinline__ constexpr uint32_t instr_desc() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOKN >> 3) << 17) |
-         ((uint32_t)(M >> 4) << 24);
-}
-
-// Order in which the CTAs take the output tiles: eight token tiles against every weight tile before the next eight, token tiles first. In
-// blockIdx order a wave of 148 CTAs would meet nearly all weight tiles with one token tile, and a matrix larger than L2 would come from HBM
-// again for every 256 tokens; like this a wave works on about as many tokens as weight rows.
-struct TileXy {
-  uint32_t x, y;
-};
-constexpr uint32_t kRasterTokens = 8;
-__device__ __forceinline__ TileXy raster(uint32_t id, uint32_t tiles_x, uint32_t tiles_y) {
-  const uint32_t first = id / (kRasterTokens * tiles_x) * kRasterTokens, in = id - first * tiles_x, tall = min(kRasterTokens, tiles_y - first);
-  return {in / tall, first + in % tall};
-}
-
 // ACT: the epilogue stores activations (kGemmGelu, kGemmRelu2, kGemmGeglu, kGemmStore); else f32 partials, or SwiGLU where `act` is given. A
 // template parameter, since the larger epilogue costs the weight-streaming shapes 0.8 us per launch.
 template <int TOKN, int WST, int XST, int MT, bool ACT>
@@ -305,7 +181,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t idesc = instr_desc<TOKN>();
+      constexpr uint32_t id = idesc(kTileN, TOKN, false);
       for (uint32_t i = 0; i < my_kb; ++i) {
         const uint32_t sw = i % WST, sx = i % XST;
         if (!mbar_wait(&full_w[sw], (i / WST) & 1)) { ok = false; break; }
@@ -317,11 +193,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
         for (int k = 0; k < kSlabK / kUmmaK; ++k) {
           // advancing 16 k elements inside the swizzle atom = +32 bytes on the start address
-          const uint64_t b = smem_desc_sw128(xt + k * kUmmaK * 2);
+          const uint64_t b = desc_k_sw128(xt + k * kUmmaK * 2);
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) {  // one accumulator of TOKN columns per weight tile
-            const uint64_t a = smem_desc_sw128(wt + mt * (kTileN * kSlabK * 2) + k * kUmmaK * 2);
-            umma_bf16(tmem_base + (uint32_t)(mt * TOKN), a, b, idesc, (i > 0 || k > 0) ? 1u : 0u);
+            const uint64_t a = desc_k_sw128(wt + mt * (kTileN * kSlabK * 2) + k * kUmmaK * 2);
+            umma_bf16(tmem_base + (uint32_t)(mt * TOKN), a, b, id, (i > 0 || k > 0) ? 1u : 0u);
           }
         }
         umma_commit(&empty_w[sw]);  // both stages are free once these MMAs have read them
@@ -473,259 +349,76 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   if (warp == 1) tmem_dealloc(tmem_base, Cfg::kTmemCols);
 }
 
-// ---- many rows: persistent CTA pairs ---------------------------------------------
-// Prompts and continuous batching (more than 256 rows) are bound by the tensor cores, with the rate at which operands reach shared memory close
-// behind. Two CTAs of a cluster work as one MMA unit (tcgen05 cta_group::2) on a tile of 256 weight rows x `tokn` tokens: each loads its own 128
-// weight rows and HALF of the token rows, so a k slab costs 32 KiB of loads per CTA for 4.2 MFLOP. The accumulator takes 256 of the 512 columns of
-// tensor memory; there are two, and the pairs stay on their SMs and go from tile to tile: the epilogue of one tile (the conversion of SwiGLU, 128 KiB
-// of f32 stores) runs under the main loop of the next, and the rings never drain in between. Tiles in the order of raster().
-struct PairConfig {
-  static constexpr int kMaxTokens = 256, kStages = 3, kStageK = 2 * kSlabK;
-  static constexpr int kWSlab = kTileN * kSlabK * 2, kXSlab = kMaxTokens / 2 * kSlabK * 2;  // 64 k of either operand
-  static constexpr int kWBytes = 2 * kWSlab, kXBytes = 2 * kXSlab;                          // one stage of either ring
-  static constexpr int kXRingOffset = kStages * kWBytes, kBarrierOffset = kXRingOffset + kStages * kXBytes;
-  static constexpr int kTmemCols = 512;
-  static constexpr int kSmemBytes = kBarrierOffset + 1024 /*align*/ + 512 /*barriers*/;
-  static constexpr uint32_t kEpilogueWarps = 4;
-};
+// ---- many rows: persistent CTA pairs (gemm_pair.cuh) ------------------------------
+
 enum PairOutput : int { kPairPartials = 0, kPairSwiglu = 1, kPairAct = 2 };
 
-struct PairTile {
-  uint32_t n0, t0, split;
-};
-// Tile `id` of the launch: the k split slowest.
-__device__ __forceinline__ PairTile pair_tile_at(uint32_t id, uint32_t tiles_x, uint32_t tiles_y, uint32_t tokn) {
-  const uint32_t plane = tiles_x * tiles_y;
-  const TileXy t = raster(id % plane, tiles_x, tiles_y);
-  return {t.x * (2 * kTileN), t.y * tokn, id / plane};
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
-}
+template <int OUT>
+struct ProjectionWork {
+  static constexpr uint32_t kBatch = 4;
+  static constexpr bool kStaticTiles = true;
+  struct Job : PairJob {
+    float *out;
+  };
+  const CUtensorMap *map_w, *map_x;
+  float *partial;
+  bf16 *act;
+  const float *bias;
+  uint32_t M, N, splits, tokn, ldc, epilogue, tiles_x, tiles_y, stages;
 
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
-// Arrives on this barrier in both CTAs of the pair once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit_both(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"((uint16_t)3)
-               : "memory");
-}
+  __device__ __forceinline__ uint32_t total() const { return tiles_x * tiles_y * splits; }
+  __device__ __forceinline__ uint32_t x_box() const { return tokn / 2; }
+  __device__ __forceinline__ bool early(uint32_t) const { return true; }
+  __device__ __forceinline__ Job job(uint32_t id) const {  // the k split slowest
+    const uint32_t plane = tiles_x * tiles_y, split = id / plane;
+    const TileXy t = raster(id % plane, tiles_x, tiles_y);
+    return {{map_w, map_x, t.x * (2 * kTileN), t.y * tokn, tokn, (uint32_t)((uint64_t)split * stages / splits), (uint32_t)((uint64_t)(split + 1) * stages / splits)},
+            partial + (size_t)split * M * N};
+  }
+  __device__ __forceinline__ void store(const Job &j, uint32_t row, uint32_t c, uint32_t (&r)[16]) const {
+    const uint32_t n = j.w_row + row, t0 = j.x_row + c;
+    if (t0 >= M) return;  // warp-uniform
+    if (OUT == kPairPartials) {
+      if (n < N) {
+#pragma unroll
+        for (uint32_t i = 0; i < 16; ++i)
+          if (t0 + i < M) j.out[(size_t)(t0 + i) * ldc + n] = __uint_as_float(r[i]);
+      }
+    } else if (OUT == kPairSwiglu || epilogue == kGemmGeglu) {
+      // Weight rows are interleaved: lane 2i holds gate f, lane 2i + 1 up f of these 16 tokens. The lanes of a pair trade halves and each
+      // finishes one token of every two (SwiGLU: tensor.rs:167-189).
+      const uint32_t odd = row & 1u, stride = OUT == kPairSwiglu ? N >> 1 : ldc;
+      bf16 *out = act + (size_t)t0 * stride + (n >> 1);
+#pragma unroll
+      for (uint32_t jj = 0; jj < 8; ++jj) {
+        const uint32_t recv = __shfl_xor_sync(0xffffffffu, odd ? r[2 * jj] : r[2 * jj + 1], 1), i = 2 * jj + odd;
+        const float g = __uint_as_float(odd ? recv : r[2 * jj]), u = __uint_as_float(odd ? r[2 * jj + 1] : recv);
+        const float v = OUT == kPairSwiglu ? __fmul_rn(g / (1.0f + __expf(-g)), u) : gelu_tanh<bf16>(g) * u;
+        if (t0 + i < M && n < N) out[(size_t)i * stride] = __float2bfloat16_rn(v);
+      }
+    } else if (n < N) {
+      bf16 *out = act + (size_t)t0 * ldc + n;
+      const float b = bias ? bias[n] : 0.f;
+#pragma unroll
+      for (uint32_t i = 0; i < 16; ++i) {
+        const float v = __uint_as_float(r[i]) + b;
+        if (t0 + i < M) out[(size_t)i * ldc] = __float2bfloat16_rn(epilogue == kGemmGelu ? gelu_tanh<bf16>(v) : (epilogue == kGemmRelu2 ? relu2(v) : v));
+      }
+    }
+  }
+};
 
 template <int OUT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(PairConfig::kThreads)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, float *__restrict__ partial,
                  bf16 *__restrict__ act, uint32_t M, uint32_t N, uint32_t K, uint32_t splits, uint32_t tokn, uint32_t ldc, uint32_t epilogue,
                  ReadyWait ready, const float *__restrict__ bias) {
-  using Cfg = PairConfig;
-  constexpr uint32_t kStages = Cfg::kStages;
-  extern __shared__ uint8_t raw_smem[];
-  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
-  uint8_t *w_ring = smem, *x_ring = smem + Cfg::kXRingOffset;
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + Cfg::kBarrierOffset);
-  uint64_t *empty = full + kStages, *acc_full = empty + kStages, *acc_empty = acc_full + 2;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
-
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = blockIdx.x & 1u, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  const bool leader = rank == 0;
-  const uint32_t nkb = (K + Cfg::kStageK - 1) / Cfg::kStageK;
-  const uint32_t tiles_x = (N + 2 * kTileN - 1) / (2 * kTileN), tiles_y = (M + tokn - 1) / tokn, total = tiles_x * tiles_y * splits;
-  auto slab_begin = [&](uint32_t split) { return (uint32_t)((uint64_t)split * nkb / splits); };
-
-  pdl_trigger();
-  if (threadIdx.x == 0) {
-    for (uint32_t s = 0; s < kStages; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 2 * Cfg::kEpilogueWarps);  // both CTAs' epilogues (used in the leader)
-    }
-    mbar_fence_init();
-  }
-  if (warp == 1) {
-    tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);
-    tmem_relinquish_pair();
-  }
-  tc_fence_before();
-  __syncthreads();
-  cluster_arrive_release();  // the peer's barriers exist before anything of this CTA signals them
-  cluster_wait_acquire();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  bool ok = true;
-
-  if (warp == 0) {
-    // Producer: this CTA's weight rows and its half of the token rows; the bytes of both CTAs are counted on the leader's barrier. Weights are
-    // immutable: those of the first slabs are asked for before the wait for the kernel that makes the activations.
-    // The whole warp runs the loop and one elected lane issues, here and below: addresses and descriptors stay in uniform registers.
-    const uint32_t half = tokn / 2, x_bytes = 2 * half * kSlabK * 2;
-    const bool elected = elect_one();
-    uint32_t it = 0, early = 0;
-    auto load_w = [&](uint32_t s, uint32_t kb, uint32_t n0) {
-      if (!elected) return;
-      const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
-      if (leader) mbar_arrive_expect_tx(&full[s], 2 * (Cfg::kWBytes + x_bytes));
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        tma_load_2d_pair(w_ring + s * Cfg::kWBytes + j * Cfg::kWSlab, &map_w, (int)(kb * Cfg::kStageK + j * kSlabK), (int)(n0 + rank * kTileN), bar);
-    };
-    {
-      const PairTile tile = pair_tile_at(pair, tiles_x, tiles_y, tokn);
-      for (uint32_t kb = slab_begin(tile.split), end = slab_begin(tile.split + 1); kb < end && early < kStages; ++kb, ++early) load_w(early, kb, tile.n0);
-    }
-    if (ready.counter) {
-      if (!wait_ready(ready)) atomicOr(&g_gemm_error, 2u);
-      fence_proxy_async_all();
-    } else {
-      pdl_wait();
-    }
-    for (uint32_t t = pair; ok && t < total; t += pairs) {
-      const PairTile tile = pair_tile_at(t, tiles_x, tiles_y, tokn);
-      for (uint32_t kb = slab_begin(tile.split), end = slab_begin(tile.split + 1); kb < end; ++kb, ++it) {
-        const uint32_t s = it % kStages;
-        if (it >= early) {
-          if (!mbar_wait(&empty[s], ((it / kStages) & 1) ^ 1)) { ok = false; break; }
-          load_w(s, kb, tile.n0);
-        }
-        if (elected) {
-          const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-            tma_load_2d_pair(x_ring + s * Cfg::kXBytes + j * Cfg::kXSlab, &map_x, (int)(kb * Cfg::kStageK + j * kSlabK), (int)(tile.t0 + rank * half), bar);
-        }
-        __syncwarp();
-      }
-    }
-    // the slots that are still being read: nobody signals a barrier of a CTA that is gone
-    for (uint32_t i = it > kStages ? it - kStages : 0; ok && i < it; ++i) ok = mbar_wait(&empty[i % kStages], (i / kStages) & 1);
-  } else if (warp == 1) {
-    if (leader) {  // the leader issues for both CTAs
-      const uint32_t idesc = instr_desc<0, 2 * kTileN>() | ((tokn >> 3) << 17);
-      const uint64_t w_desc = smem_desc_sw128(smem_u32(w_ring)), x_desc = smem_desc_sw128(smem_u32(x_ring));
-      const bool elected = elect_one();
-      uint32_t it = 0, turn = 0;
-      for (uint32_t t = pair; ok && t < total; t += pairs, ++turn) {
-        const PairTile tile = pair_tile_at(t, tiles_x, tiles_y, tokn);
-        const uint32_t buf = turn & 1, acc = tmem_base + buf * Cfg::kMaxTokens;
-        if (!mbar_wait(&acc_empty[buf], ((turn >> 1) & 1) ^ 1)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t begin = slab_begin(tile.split), end = slab_begin(tile.split + 1);
-        for (uint32_t kb = begin; kb < end; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          if (!mbar_wait(&full[s], (it / kStages) & 1)) { ok = false; break; }
-          tc_fence_after();
-          if (elected) {
-            const uint64_t a = w_desc + s * (Cfg::kWBytes >> 4), b = x_desc + s * (Cfg::kXBytes >> 4);
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-              for (int k = 0; k < kSlabK / kUmmaK; ++k)  // 16 k elements inside the swizzle atom = 32 bytes on the start address
-                umma_bf16_pair(acc, a + (j * Cfg::kWSlab + k * kUmmaK * 2 >> 4), b + (j * Cfg::kXSlab + k * kUmmaK * 2 >> 4), idesc,
-                               (kb > begin || j > 0 || k > 0) ? 1u : 0u);
-            umma_commit_both(&empty[s]);  // the stage of both CTAs is free once these MMAs have read it
-          }
-          __syncwarp();
-        }
-        if (ok && elected) umma_commit_both(&acc_full[buf]);
-      }
-    }
-  } else if (warp >= 4) {
-    // Epilogue: warp w reads tensor-memory lanes 32 * (w % 4) .. + 31 (lane = weight row, column = token).
-    const uint32_t lq = warp & 3;
-    // The output may still be read by the kernel before the producer of x. (With a ready counter the producer has read it before it counted.)
-    if (!ready.counter) pdl_wait();
-    constexpr uint32_t kBatch = 4;  // 16-column loads in flight before one wait
-    uint32_t turn = 0;
-    for (uint32_t t = pair; ok && t < total; t += pairs, ++turn) {
-      const PairTile tile = pair_tile_at(t, tiles_x, tiles_y, tokn);
-      const uint32_t buf = turn & 1, acc = tmem_base + ((lq * 32u) << 16) + buf * Cfg::kMaxTokens;
-      const uint32_t n = tile.n0 + rank * kTileN + lq * 32 + lane, t0 = tile.t0;
-      if (!mbar_wait(&acc_full[buf], (turn >> 1) & 1)) { ok = false; break; }
-      tc_fence_after();
-      float *dst = partial + (size_t)tile.split * M * N;
-      const float b_n = OUT == kPairAct && bias && n < N ? bias[n] : 0.f;
-#pragma unroll 1
-      for (uint32_t mb = 0; mb < tokn; mb += 16 * kBatch) {
-        uint32_t rr[kBatch][16];
-#pragma unroll
-        for (uint32_t b = 0; b < kBatch; ++b)
-          if (mb + 16 * b < tokn) tmem_ld16(acc + mb + 16 * b, rr[b]);
-        tmem_ld_wait();
-        if (mb + 16 * kBatch >= tokn) {  // the last of this accumulator is in registers: the MMAs of the tile after the next may write it
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[buf]), 0));
-        }
-#pragma unroll
-        for (uint32_t b = 0; b < kBatch; ++b) {
-          const uint32_t c = mb + 16 * b;
-          if (c >= tokn || t0 + c >= M) continue;  // warp-uniform
-          uint32_t (&r)[16] = rr[b];
-          if (OUT == kPairPartials) {
-            if (n < N) {
-#pragma unroll
-              for (uint32_t j = 0; j < 16; ++j)
-                if (t0 + c + j < M) dst[(size_t)(t0 + c + j) * ldc + n] = __uint_as_float(r[j]);
-            }
-          } else if (OUT == kPairSwiglu || epilogue == kGemmGeglu) {
-            // Weight rows are interleaved: lane 2i holds gate f, lane 2i + 1 up f of these 16 tokens. The lanes of a pair trade halves and each
-            // finishes one token of every two (SwiGLU: tensor.rs:167-189).
-            const uint32_t odd = lane & 1u, stride = OUT == kPairSwiglu ? N >> 1 : ldc;
-            bf16 *out = act + (size_t)(t0 + c) * stride + (n >> 1);
-#pragma unroll
-            for (uint32_t jj = 0; jj < 8; ++jj) {
-              const uint32_t recv = __shfl_xor_sync(0xffffffffu, odd ? r[2 * jj] : r[2 * jj + 1], 1), j = 2 * jj + odd;
-              const float g = __uint_as_float(odd ? recv : r[2 * jj]), u = __uint_as_float(odd ? r[2 * jj + 1] : recv);
-              const float v = OUT == kPairSwiglu ? __fmul_rn(g / (1.0f + __expf(-g)), u) : gelu_tanh<bf16>(g) * u;
-              if (t0 + c + j < M && n < N) out[(size_t)j * stride] = __float2bfloat16_rn(v);
-            }
-          } else if (n < N) {
-            bf16 *out = act + (size_t)(t0 + c) * ldc + n;
-#pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) {
-              const float v = __uint_as_float(r[j]) + b_n;
-              if (t0 + c + j < M) out[(size_t)j * ldc] = __float2bfloat16_rn(epilogue == kGemmGelu ? gelu_tanh<bf16>(v) : (epilogue == kGemmRelu2 ? relu2(v) : v));
-            }
-          }
-        }
-      }
-    }
-  }
-  if (!ok) atomicOr(&g_gemm_error, 1u);
-  tc_fence_before();
-  __syncthreads();
-  // Neither CTA leaves, nor frees the tensor memory the pair allocated together, while the other may still be read by an MMA or be reading
-  // its accumulator.
-  cluster_arrive_release();
-  cluster_wait_acquire();
-  if (warp == 1) tmem_dealloc_pair(tmem_base, Cfg::kTmemCols);
+  const ProjectionWork<OUT> work{&map_w, &map_x, partial, act, bias, M, N, splits, tokn, ldc, epilogue, (N + 2 * kTileN - 1) / (2 * kTileN),
+                                 (M + tokn - 1) / tokn, (K + PairConfig::kStageK - 1) / PairConfig::kStageK};
+  run_pairs(work, ready, &g_gemm_error);
 }
 
 // ---- host side -----------------------------------------------------------------
-
-using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                              const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                              const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeFn encode_fn() {
-  static EncodeFn fn = [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) !=
-            cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return (EncodeFn) nullptr;
-    return (EncodeFn)p;
-  }();
-  return fn;
-}
 
 // [rows][k] bf16 matrix with row stride ld; box = 64 k x box_rows, 128-byte swizzle.
 int make_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k, uint64_t ld,
@@ -813,7 +506,6 @@ int launch_tc(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float *p
 // with 256 tokens, 162 with 128, few tiles at work), and with all pairs at work the loads of 256 + tokn rows, which reach shared memory at 14 TB/s in
 // all (359-399 ns with 256 tokens, 285-308 with 192, 240-255 with 128). About 3 us for the last tile's epilogue; the consumer reads every k split's
 // slab again. Against a sweep of 22 shapes of 300 to 7006 rows, every tile and 1 to 4 splits, the choice is 1.8 % off the best on average.
-constexpr uint32_t kPairs = 74;
 uint32_t pair_tiles(uint32_t rows, uint32_t n, uint32_t tokn) { return (n + 2 * kTileN - 1) / (2 * kTileN) * ((rows + tokn - 1) / tokn); }
 uint64_t pair_cost(uint32_t rows, uint32_t n, uint32_t k, uint32_t splits, uint32_t tokn) {
   const uint64_t stages = (k + PairConfig::kStageK - 1) / PairConfig::kStageK, slabs = 2 * ((stages + splits - 1) / splits);
@@ -847,7 +539,6 @@ int launch_pair_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, f
   if (ldc != n && (splits != 1 || epi == kGemmSwiglu))
     return set_error(ORION_ERR_INTERNAL, "a strided GEMM output needs one k split and no SwiGLU");
   using Cfg = PairConfig;
-  static_assert(Cfg::kSmemBytes <= 232448, "ring exceeds the shared memory of an SM");
   static bool attr_set[kMaxDeviceOrdinals] = {};
   ORION_CUDA_CHECK("gemm_pair attr", ensure_dynamic_smem(gemm_pair_kernel<OUT>, Cfg::kSmemBytes, attr_set));
   const uint32_t tokn = pair_tokens(rows, n, k, splits);
@@ -855,7 +546,7 @@ int launch_pair_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, f
   ORION_TRY(cached_map(w, n, k, ldw, kTileN, &mw));
   ORION_TRY(cached_map(x, rows, k, ldx, tokn / 2, &mx));
   const uint32_t tiles = pair_tiles(rows, n, tokn) * splits;
-  ORION_CUDA_CHECK("gemm_pair", launch_pdl_cluster(gemm_pair_kernel<OUT>, dim3(2 * std::min(tiles, kPairs)), dim3(kThreads), dim3(2, 1, 1), Cfg::kSmemBytes,
+  ORION_CUDA_CHECK("gemm_pair", launch_pdl_cluster(gemm_pair_kernel<OUT>, dim3(2 * std::min(tiles, kPairs)), dim3(Cfg::kThreads), dim3(2, 1, 1), Cfg::kSmemBytes,
                                                    stream, *mw, *mx, partial, act, rows, n, k, splits, tokn, ldc, (uint32_t)epi, ready, bias));
   count_launch();
   ORION_CUDA_CHECK("gemm_pair", cudaGetLastError());

@@ -10,8 +10,7 @@
 //   warps 4-7  epilogue (all eight warps where an activation is computed): f32 rows, or f(w g) * (w u), f a gated activation, of neighbouring gate and up rows with the row's score w, or
 //              an activation f(w u) without a gate
 // Every wait is bounded; a wait that runs out sets the device error word and the CTA still frees its tensor memory.
-#include "kernels.h"
-#include "tcgen05.cuh"
+#include "gemm_pair.cuh"
 
 #include <algorithm>
 #include <map>
@@ -43,6 +42,49 @@ struct TcArgs {
   float *out, *shared_out;
   GatedAct f, shared_f;
 };
+
+// What a warp does with 16 rows c .. c + 15 of a tile: lane = weight row nn, r = the f32 products. GATED: see below.
+template <int GATED>
+__device__ __forceinline__ void store_chunk(const TcArgs &a, bool shared, const MoeTile &tile, uint32_t n, uint32_t nn, uint32_t c, uint32_t (&r)[16],
+                                            uint32_t split) {
+  bf16 *act = shared ? a.shared_act : a.act;
+  if (GATED == 3) {
+    bf16 v[16], *to = act + (size_t)(tile.row + c) * n + nn;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float w = shared || !a.row_score ? 1.f : a.row_score[tile.row + min(c + j, tile.count - 1)];
+      v[j] = __float2bfloat16_rn(gelu_erf<bf16>(w * __uint_as_float(r[j])));
+    }
+    if (nn < n) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j, to += n)
+        if (c + j < tile.count) *to = v[j];
+    }
+  } else if (GATED) {
+    // lane 2i holds gate f, lane 2i + 1 up f, of the same f for these 16 rows; a pair trades halves and each
+    // finishes one row of every two
+    const uint32_t odd = nn & 1u, f = nn >> 1, ffn = n >> 1;
+    bf16 v[8], *to = act + (size_t)(tile.row + c + odd) * ffn + f;
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj) {
+      const uint32_t send = odd ? r[2 * jj] : r[2 * jj + 1];
+      const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
+      const float w = shared || !a.row_score ? 1.f : a.row_score[tile.row + min(c + 2 * jj + odd, tile.count - 1)];
+      const float g = w * __uint_as_float(odd ? recv : r[2 * jj]), u = w * __uint_as_float(odd ? r[2 * jj + 1] : recv);
+      v[jj] = __float2bfloat16_rn(GATED == 1 ? silu_for<bf16>(g) * u : gated<bf16>(shared ? a.shared_f : a.f, g, u));
+    }
+    if (nn < n) {
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj, to += 2 * (size_t)ffn)
+        if (c + 2 * jj + odd < tile.count) *to = v[jj];
+    }
+  } else if (nn < n) {
+    float *out = shared ? a.shared_out + (size_t)split * a.rows * n : a.out + (size_t)split * a.sorted_rows * n;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (c + j < tile.count) out[(size_t)(tile.row + c + j) * n + nn] = __uint_as_float(r[j]);
+  }
+}
 
 // GATED: 0 = f32 products, 1 = SwiGLU, 2 = the gated activations of the arguments, 3 = no gate, the exact GELU of every product.
 template <int TOKN, int WST, int XST, int MT, int GATED>
@@ -141,8 +183,6 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     if (my_kb > 0 && !mbar_wait(acc_ready, 0)) ok = false;
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
-    float *out = shared ? a.shared_out + (size_t)split * a.rows * n : a.out + (size_t)split * a.sorted_rows * n;
-    bf16 *act = shared ? a.shared_act : a.act;
     constexpr int kBatch = TOKN >= 64 ? (GATED ? 2 : 4) : (GATED ? 1 : TOKN / 16);
 #pragma unroll 1
     for (int mb = kGroups == 2 && warp < 4 ? 16 * kBatch : 0; mb < MT * TOKN; mb += 16 * kBatch * kGroups) {
@@ -162,41 +202,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int mc = mb + 16 * b;
         const uint32_t c = mc % TOKN, nn = n0 + (mc / TOKN) * kTileN + lq * 32 + lane;  // first row of the tile in this chunk, weight row
         if (c >= tile.count) continue;  // warp-uniform
-        if (GATED == 3) {
-          bf16 v[16], *to = act + (size_t)(tile.row + c) * n + nn;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float w = shared || !a.row_score ? 1.f : a.row_score[tile.row + min(c + j, tile.count - 1)];
-            v[j] = __float2bfloat16_rn(gelu_erf<bf16>(w * __uint_as_float(rr[b][j])));
-          }
-          if (nn < n) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j, to += n)
-              if (c + j < tile.count) *to = v[j];
-          }
-        } else if (GATED) {
-          // lane 2i holds gate f, lane 2i + 1 up f, of the same f for these 16 rows; a pair trades halves and each
-          // finishes one row of every two
-          const uint32_t odd = lane & 1u, f = nn >> 1, ffn = n >> 1;
-          bf16 v[8], *to = act + (size_t)(tile.row + c + odd) * ffn + f;
-#pragma unroll
-          for (int jj = 0; jj < 8; ++jj) {
-            const uint32_t send = odd ? rr[b][2 * jj] : rr[b][2 * jj + 1];
-            const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
-            const float w = shared || !a.row_score ? 1.f : a.row_score[tile.row + min(c + 2 * jj + odd, tile.count - 1)];
-            const float g = w * __uint_as_float(odd ? recv : rr[b][2 * jj]), u = w * __uint_as_float(odd ? rr[b][2 * jj + 1] : recv);
-            v[jj] = __float2bfloat16_rn(GATED == 1 ? silu_for<bf16>(g) * u : gated<bf16>(shared ? a.shared_f : a.f, g, u));
-          }
-          if (nn < n) {
-#pragma unroll
-            for (int jj = 0; jj < 8; ++jj, to += 2 * (size_t)ffn)
-              if (c + 2 * jj + odd < tile.count) *to = v[jj];
-          }
-        } else if (nn < n) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (c + j < tile.count) out[(size_t)(tile.row + c + j) * n + nn] = __uint_as_float(rr[b][j]);
-        }
+        store_chunk<GATED>(a, shared, tile, n, nn, c, rr[b], split);
       }
     }
   }
@@ -204,6 +210,57 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, Cfg::kTmemCols);
+}
+
+// ---- tiles of 256 rows: persistent CTA pairs (gemm_pair.cuh) ------------------------
+// A prompt's products are bound by the tensor cores like its projections, and the tiles of the list are of unequal size: the pairs go from tile to tile,
+// entries without rows cost nothing and a tile with fewer rows takes as many columns as it has (in sixteens). Measured against one CTA per two weight
+// tiles and 256 rows, up and down: 7006 rows, width 2048, 16 experts of 1408 and a shared one of 2816: 343 + 160 -> 210 + 131 us; 2048 rows, experts
+// of 2112 without gates, a shared one of 4224: 115 + 80 -> 78 + 71.
+template <int GATED>
+struct MixtureWork {
+  static constexpr uint32_t kBatch = GATED ? 2 : 4;
+  static constexpr bool kStaticTiles = false;
+  struct Job : PairJob {
+    MoeTile tile;
+    uint32_t n, n0;
+    bool shared;
+  };
+  const CUtensorMap *map_w, *map_x, *map_sw, *map_sx;
+  TcArgs a;
+  uint32_t list;  // entries of the tile list
+
+  // The shared expert's tiles first, then those of the list; each as wide as its own product.
+  __device__ __forceinline__ static uint32_t wide(uint32_t n) { return (n + 2 * PairConfig::kRows - 1) / (2 * PairConfig::kRows); }
+  __device__ __forceinline__ uint32_t shared_total() const { return a.shared_tiles * wide(a.shared_n); }
+  __device__ __forceinline__ uint32_t total() const { return shared_total() + list * wide(a.n); }
+  __device__ __forceinline__ uint32_t x_box() const { return PairConfig::kMaxTokens / 2; }
+  __device__ __forceinline__ bool early(uint32_t id) const { return id < shared_total(); }
+  __device__ __forceinline__ Job job(uint32_t id) const {
+    constexpr uint32_t kRows = PairConfig::kMaxTokens;
+    const uint32_t before = shared_total();
+    Job j;
+    j.shared = id < before;
+    j.n = j.shared ? a.shared_n : a.n;
+    const TileXy t = j.shared ? raster(id, wide(j.n), a.shared_tiles) : raster(id - before, wide(j.n), list);
+    j.tile = j.shared ? MoeTile{0, t.y * kRows, min(kRows, a.rows - t.y * kRows)} : a.tiles[t.y];
+    j.n0 = t.x * 2 * PairConfig::kRows;
+    j.w = j.shared ? map_sw : map_w, j.x = j.shared ? map_sx : map_x;
+    j.w_row = j.tile.expert * j.n + j.n0;  // weight rows past the matrix read as zeros, rows past the expert belong to the next one
+    j.x_row = j.tile.row, j.cols = (j.tile.count + 15) / 16 * 16;
+    j.kb = 0, j.end = j.tile.count > 0 ? ((j.shared ? a.shared_k : a.k) + PairConfig::kStageK - 1) / PairConfig::kStageK : 0;
+    return j;
+  }
+  __device__ __forceinline__ void store(const Job &j, uint32_t row, uint32_t c, uint32_t (&r)[16]) const {
+    store_chunk<GATED>(a, j.shared, j.tile, j.n, j.n0 + row, c, r, 0);
+  }
+};
+
+template <int GATED>
+__global__ void __launch_bounds__(PairConfig::kThreads)
+moe_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_sw,
+                const __grid_constant__ CUtensorMap map_sx, TcArgs a, uint32_t list) {
+  run_pairs(MixtureWork<GATED>{&map_w, &map_x, &map_sw, &map_sx, a, list}, ReadyWait{}, &g_moe_error);
 }
 
 // [rows][k] bf16, box of 64 k x box_rows, 128-byte swizzle.
@@ -230,6 +287,10 @@ int matrix_map(const bf16 *base, uint64_t rows, uint64_t k, uint32_t box_rows, c
   return ORION_OK;
 }
 
+int product_form(const MoeProduct &p, bool gated) {
+  return !gated ? 0 : (p.f.plain() ? 3 : (p.f.kind == kGatedSilu && p.shared_f.kind == kGatedSilu ? 1 : 2));
+}
+
 template <int TOKN, int WST, int XST, int MT>
 int launch_product(const MoeProduct &p, bool swiglu, uint32_t splits, MoePlan plan, cudaStream_t stream) {
   using Cfg = MoeConfig<TOKN, WST, XST, MT>;
@@ -245,7 +306,7 @@ int launch_product(const MoeProduct &p, bool swiglu, uint32_t splits, MoePlan pl
   const TcArgs a{p.n, p.k, p.shared_n, p.shared_k, shared_tiles, p.rows, p.sorted_rows, splits, p.tiles, p.row_score, p.act, p.shared_act, p.out, p.shared_out, p.f, p.shared_f};
   const dim3 grid((std::max(p.n, p.shared_n) + MT * kTileN - 1) / (MT * kTileN), shared_tiles + plan.tiles, splits);
   static bool attr_set[4][kMaxDeviceOrdinals] = {};
-  const int form = !swiglu ? 0 : (p.f.plain() ? 3 : (p.f.kind == kGatedSilu && p.shared_f.kind == kGatedSilu ? 1 : 2));
+  const int form = product_form(p, swiglu);
   auto kernel = form == 0   ? moe_gemm_tc_kernel<TOKN, WST, XST, MT, 0>
                 : form == 1 ? moe_gemm_tc_kernel<TOKN, WST, XST, MT, 1>
                 : form == 2 ? moe_gemm_tc_kernel<TOKN, WST, XST, MT, 2>
@@ -254,6 +315,31 @@ int launch_product(const MoeProduct &p, bool swiglu, uint32_t splits, MoePlan pl
   ORION_CUDA_CHECK("moe_gemm", launch_pdl(kernel, grid, dim3(kThreads), (size_t)Cfg::kSmemBytes, stream, *mw, *mx, *msw, *msx, a));
   count_launch();
   ORION_CUDA_CHECK("moe_gemm", cudaGetLastError());
+  return ORION_OK;
+}
+
+int launch_pairs(const MoeProduct &p, bool gated, uint32_t splits, MoePlan plan, cudaStream_t stream) {
+  constexpr uint32_t kRows = PairConfig::kMaxTokens, kWide = 2 * PairConfig::kRows;
+  if (plan.tile_rows != kRows || splits != 1) return set_error(ORION_ERR_INTERNAL, "pairs take tiles of 256 rows and one k split");
+  const CUtensorMap *mw, *mx, *msw, *msx;
+  ORION_TRY(matrix_map(p.w, (uint64_t)p.experts * p.n, p.k, PairConfig::kRows, &mw));
+  ORION_TRY(matrix_map(p.x, p.sorted_rows, p.k, kRows / 2, &mx));
+  msw = mw, msx = mx;
+  if (p.shared_n) {
+    ORION_TRY(matrix_map(p.shared_w, p.shared_n, p.shared_k, PairConfig::kRows, &msw));
+    ORION_TRY(matrix_map(p.shared_x, p.rows, p.shared_k, kRows / 2, &msx));
+  }
+  const uint32_t shared_tiles = p.shared_n ? (p.rows + kRows - 1) / kRows : 0;
+  const TcArgs a{p.n, p.k, p.shared_n, p.shared_k, shared_tiles, p.rows, p.sorted_rows, 1, p.tiles, p.row_score, p.act, p.shared_act, p.out, p.shared_out, p.f, p.shared_f};
+  const uint32_t total = shared_tiles * ((p.shared_n + kWide - 1) / kWide) + plan.tiles * ((p.n + kWide - 1) / kWide);
+  static bool attr_set[4][kMaxDeviceOrdinals] = {};
+  const int form = product_form(p, gated);
+  auto kernel = form == 0 ? moe_pair_kernel<0> : form == 1 ? moe_pair_kernel<1> : form == 2 ? moe_pair_kernel<2> : moe_pair_kernel<3>;
+  ORION_CUDA_CHECK("moe_pair attr", ensure_dynamic_smem(kernel, PairConfig::kSmemBytes, attr_set[form]));
+  ORION_CUDA_CHECK("moe_pair", launch_pdl_cluster(kernel, dim3(2 * std::min(total, kPairs)), dim3(PairConfig::kThreads), dim3(2, 1, 1),
+                                                  (size_t)PairConfig::kSmemBytes, stream, *mw, *mx, *msw, *msx, a, plan.tiles));
+  count_launch();
+  ORION_CUDA_CHECK("moe_pair", cudaGetLastError());
   return ORION_OK;
 }
 
@@ -271,7 +357,7 @@ int launch_moe_product_tc(const MoeProduct &p, bool swiglu, uint32_t splits, Moe
     case 32: return launch_product<32, 6, 3, 1>(p, swiglu, splits, plan, stream);
     case 64: return launch_product<64, 5, 3, 1>(p, swiglu, splits, plan, stream);
     case 128: return launch_product<128, 4, 2, 1>(p, swiglu, splits, plan, stream);
-    default: return launch_product<256, 3, 3, 2>(p, swiglu, splits, plan, stream);
+    default: return launch_pairs(p, swiglu, splits, plan, stream);
   }
 }
 

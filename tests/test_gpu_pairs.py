@@ -1,0 +1,29 @@
+"""The persistent CTA pairs that take products of more than 256 rows: edges of tiles, k remainders, k splits, one tile and several rounds."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (257, 256, 64),     # the smallest batch that takes them, half a stage of k
+    (272, 255, 72),     # rows of a tile past the matrix, k that ends inside a slab
+    (300, 384, 200),    # the second CTA of the last pair without weight rows
+    (512, 1024, 4096),  # k splits
+    (513, 130, 136),    # one row in the last token tile
+    (700, 8, 1096),     # fewer weight rows than a quarter of a warpgroup
+    (1031, 6400, 136),  # more than one round of the 74 pairs, ragged
+    (2065, 2432, 392),  # nine token tiles: a group of eight and one more
+]
+
+
+@pytest.mark.parametrize("rows,n,k", SHAPES)
+def test_products_of_many_rows(pkg, backend, rows, n, k):
+    rng = np.random.default_rng(rows * 7 + n)
+    from oracle import binding as oracle
+    x, w = (oracle.round_to_bf16(rng.standard_normal(s).astype(np.float32)) for s in ((rows, k), (n, k)))
+    got = pkg.ops.linear(backend, x, w, None, pkg.DType.BF16)
+    exact, size = x.astype(np.float64) @ w.T.astype(np.float64), np.abs(x).astype(np.float64) @ np.abs(w).T.astype(np.float64)
+    # products of bf16 are exact in f32; an MMA adds 16 of them and the accumulator, each sum cut off below 2^-23 of what stands in it at most,
+    # and a k split one rounding more
+    bound = (k / 16 + 8) * 2.0 ** -23 * size
+    assert np.all(np.abs(got - exact) <= bound), float(np.max(np.abs(got - exact) / bound))
