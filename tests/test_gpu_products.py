@@ -1,4 +1,4 @@
-"""The persistent CTA pairs that take products of more than 256 rows: edges of tiles, k remainders, k splits, one tile and several rounds."""
+"""Products at the edges of their tiles: the persistent CTA pairs of more than 256 rows (tiles, k remainders, k splits, rounds), the f32 decode kernel."""
 import numpy as np
 import pytest
 
@@ -16,6 +16,11 @@ SHAPES = [
 ]
 
 
+@pytest.fixture(scope="module")
+def backend(pkg):
+    return pkg.CudaBackend(0)
+
+
 @pytest.mark.parametrize("rows,n,k", SHAPES)
 def test_products_of_many_rows(pkg, backend, rows, n, k):
     rng = np.random.default_rng(rows * 7 + n)
@@ -27,3 +32,13 @@ def test_products_of_many_rows(pkg, backend, rows, n, k):
     # and a k split one rounding more
     bound = (k / 16 + 8) * 2.0 ** -23 * size
     assert np.all(np.abs(got - exact) <= bound), float(np.max(np.abs(got - exact) / bound))
+
+
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 64, 65])
+@pytest.mark.parametrize("n,k", [(1, 4), (17, 100), (130, 128), (16, 132), (33, 684), (15, 6)])
+def test_f32_products_of_few_rows_are_bit_exact(pkg, backend, rows, n, k):
+    """The kernel of decode batches, its neighbours in rows and k it does not take: one chain of additions per output, whatever the tile."""
+    from oracle import binding as oracle
+    rng = np.random.default_rng(rows * 7 + n + k)
+    x, w = rng.standard_normal((rows, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    assert np.array_equal(pkg.ops.linear(backend, x, w), oracle.linear(x, w))
