@@ -828,6 +828,8 @@ int launch_paged_attention_decode_form(const bf16 *q, const bf16 *arena, KvLayou
   return run(q, arena, kv, layer, batch, rows, q_heads, splits, scratch, form, out, stream);
 }
 
+const void *decode_error_word() { return device_symbol(g_decode_error); }
+
 int decode_poll_error(uint32_t *code) {
   uint32_t v = 0;
   ORION_CUDA_CHECK("decode error word", cudaMemcpyFromSymbol(&v, g_decode_error, sizeof v));

@@ -240,6 +240,8 @@ int launch_paged_attention_prefill(const bf16 *q, const bf16 *arena, KvLayout kv
   return ORION_OK;
 }
 
+const void *prefill_error_word() { return device_symbol(g_prefill_error); }
+
 int prefill_poll_error(uint32_t *code) {
   uint32_t tc = 0;
   ORION_TRY(prefill_tc_poll_error(&tc));

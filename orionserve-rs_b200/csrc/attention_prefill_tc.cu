@@ -529,6 +529,8 @@ int launch_paged_attention_prefill_form(const bf16 *q, const bf16 *arena, KvLayo
   return run(q, arena, kv, layer, batch, tiles, num_tiles, q_heads, form, out, stream);
 }
 
+const void *prefill_tc_error_word() { return device_symbol(g_prefill_tc_error); }
+
 int prefill_tc_poll_error(uint32_t *code) {
   uint32_t v = 0;
   ORION_CUDA_CHECK("prefill error word", cudaMemcpyFromSymbol(&v, g_prefill_tc_error, sizeof v));

@@ -36,6 +36,13 @@ void clear_error();
     if (_rc != ORION_OK) return _rc; \
   } while (0)
 
+// Device address of a variable on the current device; null with the error pending if there is none.
+template <typename S>
+inline const void *device_symbol(const S &symbol) {
+  void *p = nullptr;
+  return cudaGetSymbolAddress(&p, symbol) == cudaSuccess ? p : nullptr;
+}
+
 // Number of kernels launched through launch accounting since the last reset.
 extern thread_local uint64_t g_launch_count;
 inline void count_launch() { ++g_launch_count; }

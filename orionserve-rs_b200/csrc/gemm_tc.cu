@@ -651,6 +651,8 @@ int launch_gemm_tc(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, flo
   }
 }
 
+const void *gemm_tc_error_word() { return device_symbol(g_gemm_error); }
+
 int gemm_tc_poll_error(uint32_t *code) {
 #ifdef ORION_TRACE
   static const bool tracing = std::getenv("ORION_GEMM_TRACE") != nullptr &&

@@ -455,6 +455,8 @@ int launch_gla_chunks(const float *partial, uint32_t splits, size_t split_stride
   return after_launch("gla_finish");
 }
 
+const void *gla_error_word() { return device_symbol(g_gla_error); }
+
 int gla_poll_error(uint32_t *code) {
   uint32_t v = 0;
   ORION_CUDA_CHECK("gla error word", cudaMemcpyFromSymbol(&v, g_gla_error, sizeof v));

@@ -654,6 +654,24 @@ int launch_tp_allreduce_residual_rmsnorm(const TpPeers &peers, const uint32_t *e
 // state[0] += epochs (wrapped as described above), state[1] += rows_counted, after the preceding kernel has completed.
 int launch_tp_state_bump(uint32_t *state, uint32_t epochs, uint32_t rows_counted, cudaStream_t stream);
 int tp_poll_error(uint32_t *code);
+
+// The error words that bounded waits set, one per translation unit, on the current device. launch_error_words writes the OR of all of
+// them to `out`, page-locked host memory, once what the stream holds has run: a step that ends well then costs its caller no read of device memory.
+struct ErrorWords {
+  static constexpr int kWords = 9;
+  const uint32_t *word[kWords];
+};
+const void *decode_error_word();
+const void *prefill_error_word();
+const void *prefill_tc_error_word();
+const void *gemm_tc_error_word();
+const void *gla_error_word();
+const void *latent_error_word();
+const void *latent_prefill_error_word();
+const void *moe_error_word();
+const void *tp_error_word();
+int find_error_words(ErrorWords *out);
+int launch_error_words(const ErrorWords &words, uint32_t *out, cudaStream_t stream);
 // Vocabulary-parallel LM head: `launch_tp_signal` (ranks other than the leader) stores `epoch` into the
 // rank's flag in the leader's memory once the preceding kernel of the stream has completed;
 // `launch_tp_wait_flags` (leader) holds the stream until the flags of ranks 1 .. world-1 carry `epoch`

@@ -698,6 +698,8 @@ int launch_latent_decode(const bf16 *qa, const bf16 *cache, const bf16 *w_uv, co
   return after_launch("latent_value");
 }
 
+const void *latent_error_word() { return device_symbol(g_latent_error); }
+
 int latent_poll_error(uint32_t *code) {
   uint32_t v = 0;
   ORION_CUDA_CHECK("latent attention error word", cudaMemcpyFromSymbol(&v, g_latent_error, sizeof v));

@@ -358,6 +358,8 @@ int launch_latent_prefill(const bf16 *q, const bf16 *expanded, const bf16 *rotat
   return ORION_OK;
 }
 
+const void *latent_prefill_error_word() { return device_symbol(g_latent_prefill_error); }
+
 int latent_prefill_poll_error(uint32_t *code) {
   uint32_t v = 0;
   ORION_CUDA_CHECK("latent prefill error word", cudaMemcpyFromSymbol(&v, g_latent_prefill_error, sizeof v));

@@ -361,6 +361,8 @@ int launch_moe_product_tc(const MoeProduct &p, bool swiglu, uint32_t splits, Moe
   }
 }
 
+const void *moe_error_word() { return device_symbol(g_moe_error); }
+
 int moe_poll_error(uint32_t *code) {
   uint32_t v = 0;
   ORION_CUDA_CHECK("mixture error word", cudaMemcpyFromSymbol(&v, g_moe_error, sizeof v));

@@ -53,6 +53,7 @@ class StepModel : public ModelBase {
     drop_graphs();
     for (void *p : allocs_) cudaFree(p);
     if (h_meta_) cudaFreeHost(h_meta_);
+    if (h_error_) cudaFreeHost(const_cast<uint32_t *>(h_error_));
     if (stage_raw_) cudaFree(stage_raw_);
     if (stage_f32_) cudaFree(stage_f32_);
     for (cudaEvent_t e : head_ev_)
@@ -253,6 +254,8 @@ class StepModel : public ModelBase {
   cudaEvent_t head_ev_[kHeadChunks] = {};
   uint32_t head_off_[kHeadChunks] = {}, head_cols_[kHeadChunks] = {};
   int head_chunks_ = 0;
+  ErrorWords error_words_{};
+  volatile uint32_t *h_error_ = nullptr;  // page-locked; see launch_error_words
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   std::vector<void *> allocs_;
   T *embed_ = nullptr, *lm_head_ = nullptr;
@@ -293,6 +296,11 @@ int StepModel<T>::init_step(const StepShape &shape) {
   ORION_CUDA_CHECK("create stream", cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   ORION_CUDA_CHECK("create stream", cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
   for (cudaEvent_t &e : head_ev_) ORION_CUDA_CHECK("create event", cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  void *error_raw = nullptr;
+  ORION_CUDA_CHECK("allocate error word", cudaMallocHost(&error_raw, sizeof(uint32_t)));
+  h_error_ = static_cast<uint32_t *>(error_raw);
+  *h_error_ = 0;
+  ORION_TRY(find_error_words(&error_words_));
   ORION_CUDA_CHECK("create event", cudaEventCreate(&ev0_));
   ORION_CUDA_CHECK("create event", cudaEventCreate(&ev1_));
   const size_t rows = shape.max_batch_tokens, H = shape.hidden;
@@ -394,11 +402,13 @@ int StepModel<T>::run_head(bool want_argmax) {
     const float c = logit_softcap();
     return c == 0.f ? ORION_OK : timed(kProfElementwise, [&] { return launch_softcap(logits_ + n0, S, n, V, c, stream_); });
   };
-  if (kBf16 && hp.tensor_core && V >= 4 * 8192 && !want_argmax) {
-    // A large vocabulary goes out in column blocks, an event after each: forward() copies block i
-    // to the host (copy engine, second stream) while block i + 1 is being computed.
-    const uint32_t per = (((V + 127) / 128 + kHeadChunks - 1) / kHeadChunks) * 128;
-    for (uint32_t c = 0; c < (uint32_t)kHeadChunks && c * per < V; ++c) {
+  // A large vocabulary goes out in column blocks, an event after each: forward() copies block i to the host (copy engine, second stream) while block
+  // i + 1 is being computed. A block has at least 128 weight tiles: with fewer CTAs it takes as long as with one on every SM (four blocks of 64 tiles
+  // of k 4096 take 25-30 us each). Logits of up to half a MiB leave in one copy of 10 us, about what an event and a second copy cost.
+  const uint32_t tiles = (V + 127) / 128, blocks = std::min<uint32_t>(kHeadChunks, tiles / 128);
+  if (kBf16 && hp.tensor_core && V >= 4 * 8192 && !want_argmax && (size_t)S * V * sizeof(float) > (512u << 10)) {
+    const uint32_t per = (tiles + blocks - 1) / blocks * 128;
+    for (uint32_t c = 0; c < blocks && c * per < V; ++c) {
       const uint32_t n0 = c * per, nn = std::min(per, V - n0);
       GemmPlan cp = hp;
       cp.ldc = V;
@@ -559,6 +569,7 @@ int StepModel<T>::forward(const BatchView &b, float *logits_out, uint64_t logits
   ORION_CUDA_CHECK("upload batch", cudaMemcpyAsync(d_meta_, h, mt.total * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
   ORION_TRY(run_step(token_ids_out != nullptr));
   last_launches_ = g_launch_count;
+  if (DTypeOf<T>::is_bf16) ORION_TRY(launch_error_words(error_words_, const_cast<uint32_t *>(h_error_), stream_));
   if (mt.zero_count) {
     ORION_TRY(wait_for(stream_, "forward"));
     // transformer.rs:413-417: detected after the layers ran, so KV slots were written.
@@ -585,7 +596,9 @@ int StepModel<T>::forward(const BatchView &b, float *logits_out, uint64_t logits
                                                           cudaMemcpyDeviceToHost, stream_));
     ORION_TRY(wait_for(stream_, "forward"));
   }
-  ORION_TRY(poll_errors());
+  // The words of all translation units came with the step: only a wait that ran out (in whichever model) is looked into. The f32 build has none of
+  // its own, and polls what its collectives have.
+  if (!DTypeOf<T>::is_bf16 || *h_error_ != 0) ORION_TRY(poll_errors());
   step_done(b);
   return ORION_OK;
 }

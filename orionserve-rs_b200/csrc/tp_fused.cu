@@ -480,6 +480,8 @@ int selftest_peer_wait(uint64_t limit_us, uint32_t *timed_out, uint32_t *waited_
   return ORION_OK;
 }
 
+const void *tp_error_word() { return device_symbol(g_tp_error); }
+
 int tp_poll_error(uint32_t *code) {
 #ifdef ORION_TRACE
   static const bool tracing = std::getenv("ORION_TP_TRACE") != nullptr &&
