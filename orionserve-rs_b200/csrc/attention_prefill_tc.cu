@@ -9,7 +9,7 @@
 //              arena (3-D tensor maps over [chunk][slot][dim], one for K and one for V; a 16-slot x 64-dim box lands as
 //              sixteen 128-byte rows, and because the arena keeps the 16-byte groups of a row XOR-permuted
 //              by slot & 7, those rows ARE the 128-byte-swizzled operand layout the MMA expects);
-//   warp 1     allocates tensor memory; one lane issues S = Q K^T (M 128, N 64, K 128) and, once the
+//   warp 1     allocates tensor memory; one elected lane issues S = Q K^T (M 128, N 64, K 128) and, once the
 //              softmax warps have written P, O (+)= P V (M 128, N 128, K 64; V is the MN-major operand; keys
 //              that are values as well are one tile for both);
 //   warps 2-5  one thread per row: read the row of S from tensor memory (lane = row, so max and sum
@@ -39,9 +39,10 @@ constexpr int kThreads = 192;
 template <int DK, int DV, bool JOINT>
 struct PrefillTcConfig {
   // Where tensor memory has room for it without costing a CTA, S has two buffers: the scores of the next key tile are computed under
-  // the softmax of this one.
-  static constexpr bool kTwoS = JOINT && DV == 128;
-  static constexpr int kStages = kTwoS ? 3 : 2;
+  // the softmax of this one. Measured, per layer: four prompts of 2048, 32 heads over 8, 322 -> 290 us; four of 1531 to 2047, 16 over 4, windows and
+  // soft caps, 140 -> 113 (both with the longest tiles first, which alone gives 5 %).
+  static constexpr bool kTwoS = DV == 128;
+  static constexpr int kStages = JOINT && kTwoS ? 3 : 2;  // of K and V tiles; three of both would leave room for one CTA
   static constexpr uint32_t kTmemO = kTwoS ? 128 : 64;  // S: the first columns of tensor memory, O behind them
   static constexpr int kQBytes = DK / 64 * kM * 128;     // 64-dim slabs of [128 rows][128 bytes]
   static constexpr int kKBytes = DK / 64 * kKeys * 128;  // 64-dim slabs of [64 keys][128 bytes]
@@ -90,7 +91,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 
   if (!FORM) pdl_trigger();
   const uint32_t kvh = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const PrefillTile tile = tiles[blockIdx.y];
+  const PrefillTile tile = tiles[gridDim.y - 1 - blockIdx.y];  // from the end: a prompt's last tiles see the most keys, and none of them starts last
   const uint32_t group = q_heads / kv.num_kv_heads;
   const uint32_t *table = batch.tables_flat + batch.table_offsets[tile.seq];
   const uint32_t nblocks = tile.max_position / kBlk + 1;
@@ -138,71 +139,76 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 
   if (warp == 0) {
     // ---- K/V producer ----
-    if (lane == 0) {
-      pdl_wait();  // this step's K/V rows come from the preceding kernel
-      const uint32_t chunk0 = layer * kv.num_blocks;
-      for (uint32_t j = 0; j < ntiles; ++j) {
-        const uint32_t s = j % kStages, use = j / kStages;
-        if (!wait(&kv_empty[s], (use & 1) ^ 1)) { ok = false; break; }
-        mbar_arrive_expect_tx(&kv_full[s], kStageBytes + (JOINT ? kKeys * 4 : 0));
-        uint8_t *k_dst = ring + s * kStageBytes, *v_dst = k_dst + kKBytes;
+    const bool elected = elect_one();
+    pdl_wait();  // this step's K/V rows come from the preceding kernel
+    const uint32_t chunk0 = layer * kv.num_blocks;
+    for (uint32_t j = 0; j < ntiles; ++j) {
+      const uint32_t s = j % kStages, use = j / kStages;
+      if (!__all_sync(0xffffffffu, wait(&kv_empty[s], (use & 1) ^ 1))) { ok = false; break; }
+      if (!elected) continue;
+      mbar_arrive_expect_tx(&kv_full[s], kStageBytes + (JOINT ? kKeys * 4 : 0));
+      uint8_t *k_dst = ring + s * kStageBytes, *v_dst = k_dst + kKBytes;
 #pragma unroll
-        for (uint32_t b = 0; b < kKeys / kBlk; ++b) {
-          // a block past the row's context repeats the first one: its keys are masked, its values must be finite
-          const uint32_t lb = logical(j * (kKeys / kBlk) + b);
-          const uint32_t block = table[lb < nblocks ? lb : block0];
-          const int chunk = (int)((chunk0 + block) * kv.num_kv_heads + kvh);
+      for (uint32_t b = 0; b < kKeys / kBlk; ++b) {
+        // a block past the row's context repeats the first one: its keys are masked, its values must be finite
+        const uint32_t lb = logical(j * (kKeys / kBlk) + b);
+        const uint32_t block = table[lb < nblocks ? lb : block0];
+        const int chunk = (int)((chunk0 + block) * kv.num_kv_heads + kvh);
 #pragma unroll
-          for (int h = 0; h < DK / 64; ++h)
-            tma_load_3d(k_dst + h * (kKeys * 128) + b * (kBlk * 128), &map_k, h * 64, 0, chunk, &kv_full[s]);
-          if (JOINT) {
-            bulk_copy_g2s(factors + s * kKeys + b * kBlk, arena + kv.factor(layer, block, kvh, 0), kBlk * 4, &kv_full[s]);
-            continue;
-          }
-#pragma unroll
-          for (int h = 0; h < DV / 64; ++h)
-            tma_load_3d(v_dst + h * (kKeys * 128) + b * (kBlk * 128), &map_v, h * 64, 0, chunk, &kv_full[s]);
+        for (int h = 0; h < DK / 64; ++h)
+          tma_load_3d(k_dst + h * (kKeys * 128) + b * (kBlk * 128), &map_k, h * 64, 0, chunk, &kv_full[s]);
+        if (JOINT) {
+          bulk_copy_g2s(factors + s * kKeys + b * kBlk, arena + kv.factor(layer, block, kvh, 0), kBlk * 4, &kv_full[s]);
+          continue;
         }
+#pragma unroll
+        for (int h = 0; h < DV / 64; ++h)
+          tma_load_3d(v_dst + h * (kKeys * 128) + b * (kBlk * 128), &map_v, h * 64, 0, chunk, &kv_full[s]);
       }
     }
   } else if (warp == 1) {
     // ---- MMA issue ----
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = idesc(kM, kKeys, false), idesc_o = idesc(kM, DV, true);
-      const uint32_t qa = smem_u32(q_smem);
-      // S = Q K^T: 64-dim slabs, four 16-dim steps each (+32 bytes inside the swizzle atom)
-      auto scores = [&](uint32_t j) -> bool {
-        const uint32_t s = j % kStages;
-        if (!wait(&kv_full[s], (j / kStages) & 1)) return false;
-        tc_fence_after();
-        const uint32_t ka = smem_u32(ring + s * kStageBytes), b = kTwoS ? j & 1 : 0;
+    const bool elected = elect_one();
+    constexpr uint32_t idesc_s = idesc(kM, kKeys, false), idesc_o = idesc(kM, DV, true);
+    const uint64_t q_desc = desc_k_sw128(smem_u32(q_smem)), k_desc = desc_k_sw128(smem_u32(ring));
+    const uint64_t v_desc = desc_mn_sw128(smem_u32(ring) + (JOINT ? 0 : kKBytes), kKeys * 128, 1024);
+    auto arrived = [&](uint64_t *bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, wait(bar, parity)); };
+    // S = Q K^T: 64-dim slabs, four 16-dim steps each (+32 bytes inside the swizzle atom)
+    auto scores = [&](uint32_t j) -> bool {
+      const uint32_t s = j % kStages;
+      if (!arrived(&kv_full[s], (j / kStages) & 1)) return false;
+      tc_fence_after();
+      const uint32_t b = kTwoS ? j & 1 : 0;
+      if (elected) {
+        const uint64_t kd = k_desc + s * (kStageBytes >> 4);
 #pragma unroll
         for (int ks = 0; ks < DK / 16; ++ks) {
           const uint32_t h = ks >> 2, kk = ks & 3;
-          umma_bf16(tmem_base + b * kKeys, desc_k_sw128(qa + h * (kM * 128) + kk * 32), desc_k_sw128(ka + h * (kKeys * 128) + kk * 32),
-                    idesc_s, ks > 0 ? 1u : 0u);
+          umma_bf16(tmem_base + b * kKeys, q_desc + ((h * (kM * 128) + kk * 32) >> 4), kd + ((h * (kKeys * 128) + kk * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
         }
         umma_commit(&s_ready[b]);
-        return true;
-      };
-      if (!wait(q_ready, 0)) ok = false;
-      if (kTwoS && ok && ntiles > 0) ok = scores(0);
-      for (uint32_t j = 0; ok && j < ntiles; ++j) {
-        const uint32_t s = j % kStages;
-        // the other buffer's scores have been read: their P came before the product of the tile before
-        if (kTwoS ? j + 1 < ntiles && !scores(j + 1) : !scores(j)) { ok = false; break; }
-        const uint32_t ka = smem_u32(ring + s * kStageBytes), va = JOINT ? ka : ka + kKBytes;
-        if (!wait(p_ready, j & 1)) { ok = false; break; }
-        tc_fence_after();
-        // O (+)= P V: P is [128 rows][64 keys] (where the K tile was, if it fits there); V is [key][dim]: MN-major, 16 keys per step
-        const uint32_t pa = smem_u32(p_tile(s));
+      }
+      __syncwarp();
+      return true;
+    };
+    if (!arrived(q_ready, 0)) ok = false;
+    if (kTwoS && ok && ntiles > 0) ok = scores(0);
+    for (uint32_t j = 0; ok && j < ntiles; ++j) {
+      const uint32_t s = j % kStages;
+      // the other buffer's scores have been read: their P came before the product of the tile before
+      if (kTwoS ? j + 1 < ntiles && !scores(j + 1) : !scores(j)) { ok = false; break; }
+      if (!arrived(p_ready, j & 1)) { ok = false; break; }
+      tc_fence_after();
+      // O (+)= P V: P is [128 rows][64 keys] (where the K tile was, if it fits there); V is [key][dim]: MN-major, 16 keys per step
+      if (elected) {
+        const uint64_t pd = desc_k_sw128(smem_u32(p_tile(s))), vd = v_desc + s * (kStageBytes >> 4);
 #pragma unroll
         for (int ks = 0; ks < kKeys / 16; ++ks)
-          umma_bf16(tmem_base + kTmemO, desc_k_sw128(pa + ks * 32), desc_mn_sw128(va + ks * (16 * 128), kKeys * 128, 1024),
-                    idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+          umma_bf16(tmem_base + kTmemO, pd + ks * 2, vd + ks * (16 * 128 >> 4), idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
         umma_commit(o_ready);
         umma_commit(&kv_empty[s]);
       }
+      __syncwarp();
     }
   } else {
     // ---- softmax: thread = row ----
@@ -244,6 +250,9 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       sl2 = 1.f;
       fixed = cap_out <= 60.f && !form.sinks;
     }
+    // Scores stay as they are until the exponent, ex2(mul * score - reference); the maximum of what is multiplied needs a positive factor.
+    const bool flip = !JOINT && sl2 < 0.f;
+    const float mul = JOINT ? 1.f : fabsf(sl2);
     float dist_mult = 0.f, dist_rate = 0.f;
     if (JOINT && form.dist_mult) dist_mult = form.dist_mult[head], dist_rate = form.dist_rate[head];
     float ref = -INFINITY, l = 0.f;
@@ -260,6 +269,10 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       const bool straight = FORM != 2 || j * (kKeys / kBlk) >= kept_blk || kept_blk == block0;  // the tile's keys follow one another
       const int key0 = (int)(logical(j * (kKeys / kBlk)) * kBlk);
       float mx = -INFINITY;
+      if (flip) {
+#pragma unroll
+        for (int i = 0; i < kKeys; ++i) sr[i >> 5][i & 31] ^= 0x80000000u;
+      }
       if (JOINT) {
         if (!__all_sync(0xffffffffu, wait(&kv_full[s], (j / kStages) & 1))) ok = false;  // the factors landed with the tile
         const float4 *factor = reinterpret_cast<const float4 *>(factors + s * kKeys);
@@ -318,12 +331,10 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         if (FORM == 2 && fixed) {
           mx = 0.f;
         } else {
+          float most[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains
 #pragma unroll
-          for (int i = 0; i < kKeys; ++i) {
-            const float v = JOINT ? __uint_as_float(sr[i >> 5][i & 31]) : __uint_as_float(sr[i >> 5][i & 31]) * sl2;
-            sr[i >> 5][i & 31] = __float_as_uint(v);
-            mx = fmaxf(mx, v);
-          }
+          for (int i = 0; i < kKeys; ++i) most[i & 3] = fmaxf(most[i & 3], __uint_as_float(sr[i >> 5][i & 31]));
+          mx = fmaxf(fmaxf(most[0], most[1]), fmaxf(most[2], most[3])) * mul;
         }
       } else {
         int from[kKeys / kBlk];  // first key of every block
@@ -332,10 +343,11 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 #pragma unroll
         for (int i = 0; i < kKeys; ++i) {
           const int key = from[i / kBlk] + i % kBlk;
-          const float v = (key <= pos && (!FORM || key >= low || (FORM == 2 && key < keep))) ? __uint_as_float(sr[i >> 5][i & 31]) * (JOINT ? 1.f : sl2) : -INFINITY;
+          const float v = (key <= pos && (!FORM || key >= low || (FORM == 2 && key < keep))) ? __uint_as_float(sr[i >> 5][i & 31]) : -INFINITY;
           sr[i >> 5][i & 31] = __float_as_uint(v);
           mx = fmaxf(mx, v);
         }
+        mx *= mul;
       }
       if (FORM == 2 && fixed) mx = 0.f;  // the reference stays at zero: the exponents are between plus and minus the cap
       // The reference of the exponentials moves only when the maximum runs away from it.
@@ -366,17 +378,19 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       l *= corr;
       const float base = ref == -INFINITY ? 0.f : ref;
       uint8_t *p_row = p_tile(s) + m * 128;
+      float sums[4] = {l, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int c = 0; c < kKeys / 8; ++c) {
         float p[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          p[i] = ex2(__uint_as_float(sr[(c * 8 + i) >> 5][(c * 8 + i) & 31]) - base);
-          l += p[i];
+          p[i] = ex2(fmaf(__uint_as_float(sr[(c * 8 + i) >> 5][(c * 8 + i) & 31]), mul, -base));
+          sums[i & 3] += p[i];
         }
         *reinterpret_cast<uint4 *>(p_row + ((c ^ (m & 7)) << 4)) =
             make_uint4(pack2(p[0], p[1]), pack2(p[2], p[3]), pack2(p[4], p[5]), pack2(p[6], p[7]));
       }
+      l = (sums[0] + sums[1]) + (sums[2] + sums[3]);
       tc_fence_before();        // the loads of S (and the rescale of O) precede the next MMAs
       fence_proxy_async_smem();  // P was written through the generic proxy, the MMA reads it through the async proxy
       softmax_bar();

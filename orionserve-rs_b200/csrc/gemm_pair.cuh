@@ -59,11 +59,6 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
 // Arrives on this barrier in both CTAs of the pair once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit_both(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
@@ -148,6 +143,7 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
   pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
   bool ok = true;
+  auto wait = [](uint64_t *bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity)); };  // one answer for a warp
 
   if (warp == 0) {
     // Producer: this CTA's weight rows and its half of the token rows; the bytes of both CTAs are counted on the leader's barrier. Weights are
@@ -178,7 +174,7 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
       for (uint32_t kb = j.kb; kb < j.end; ++kb, ++it) {
         const uint32_t s = it % kStages;
         if (it >= early) {
-          if (!mbar_wait(&empty[s], ((it / kStages) & 1) ^ 1)) { ok = false; break; }
+          if (!wait(&empty[s], ((it / kStages) & 1) ^ 1)) { ok = false; break; }
           load_w(s, kb, j);
         }
         if (elected) {
@@ -191,7 +187,7 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
       }
     }
     // the slots that are still being read: nobody signals a barrier of a CTA that is gone
-    for (uint32_t i = it > kStages ? it - kStages : 0; ok && i < it; ++i) ok = mbar_wait(&empty[i % kStages], (i / kStages) & 1);
+    for (uint32_t i = it > kStages ? it - kStages : 0; ok && i < it; ++i) ok = wait(&empty[i % kStages], (i / kStages) & 1);
   } else if (warp == 1) {
     if (leader) {  // issues for both CTAs
       const uint64_t w_desc = desc_k_sw128(smem_u32(w_ring)), x_desc = desc_k_sw128(smem_u32(x_ring));
@@ -202,11 +198,11 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
         const typename Work::Job j = work.job(t);
         if (j.kb >= j.end) continue;
         const uint32_t id = idesc(2 * Cfg::kRows, j.cols, false), buf = turn & 1, acc = tmem_base + buf * Cfg::kMaxTokens;
-        if (!mbar_wait(&acc_empty[buf], ((turn >> 1) & 1) ^ 1)) { ok = false; break; }
+        if (!wait(&acc_empty[buf], ((turn >> 1) & 1) ^ 1)) { ok = false; break; }
         tc_fence_after();
         for (uint32_t kb = j.kb; kb < j.end; ++kb, ++it) {
           const uint32_t s = it % kStages;
-          if (!mbar_wait(&full[s], (it / kStages) & 1)) { ok = false; break; }
+          if (!wait(&full[s], (it / kStages) & 1)) { ok = false; break; }
           tc_fence_after();
           if (elected) {
             const uint64_t a = w_desc + s * (Cfg::kWBytes >> 4), b = x_desc + s * (Cfg::kXBytes >> 4);
@@ -234,7 +230,7 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
       const typename Work::Job j = work.job(t);
       if (j.kb >= j.end) continue;
       const uint32_t buf = turn & 1, acc = tmem_base + (((warp & 3) * 32u) << 16) + buf * Cfg::kMaxTokens;
-      if (!mbar_wait(&acc_full[buf], (turn >> 1) & 1)) { ok = false; break; }
+      if (!wait(&acc_full[buf], (turn >> 1) & 1)) { ok = false; break; }
       ++turn;
       tc_fence_after();
       constexpr uint32_t kStep = 16 * kBatch * (Cfg::kEpilogueWarps / 4);

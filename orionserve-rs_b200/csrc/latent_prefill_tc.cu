@@ -116,57 +116,69 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     return false;
   };
 
+  auto arrived = [&](uint64_t *bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, wait(bar, parity)); };  // one answer for a warp
+
   if (warp == 0) {
     // ---- K/V producer ----
-    if (lane == 0) {
-      pdl_wait();
-      const int row0 = tile.row_of_zero + (int)first_key;  // expanded row of the tile's first key
-      const uint32_t k_bytes = lay.slabs * kKSlab, v_bytes = lay.value_slabs * kKSlab;
-      for (uint32_t j = 0; j < ntiles; ++j) {
-        const int row = row0 + (int)(j * kKeys);
-        if (j > 0 && !wait(k_empty, (j - 1) & 1)) { ok = false; break; }
+    const bool elected = elect_one();
+    pdl_wait();
+    const int row0 = tile.row_of_zero + (int)first_key;  // expanded row of the tile's first key
+    const uint32_t k_bytes = lay.slabs * kKSlab, v_bytes = lay.value_slabs * kKSlab;
+    for (uint32_t j = 0; j < ntiles; ++j) {
+      const int row = row0 + (int)(j * kKeys);
+      if (j > 0 && !arrived(k_empty, (j - 1) & 1)) { ok = false; break; }
+      ++k_issued;
+      if (elected) {
         mbar_arrive_expect_tx(k_full, k_bytes);
-        ++k_issued;
         for (uint32_t h = 0; h < lay.dim_slabs; ++h) tma_load_3d(k_smem + h * kKSlab, &map_k, (int)(h * 64), (int)head, row, k_full);
         for (uint32_t h = lay.dim_slabs; h < lay.slabs; ++h)
           tma_load_2d(k_smem + h * kKSlab, &map_rot, (int)((h - lay.dim_slabs) * 64), row, k_full);
-        if (j > 0 && !wait(o_ready, (j - 1) & 1)) { ok = false; break; }
+      }
+      __syncwarp();
+      if (j > 0 && !arrived(o_ready, (j - 1) & 1)) { ok = false; break; }
+      ++v_issued;
+      if (elected) {
         mbar_arrive_expect_tx(v_full, v_bytes);
-        ++v_issued;
         for (uint32_t h = 0; h < lay.value_slabs; ++h) tma_load_3d(v_smem + h * kKSlab, &map_v, (int)(h * 64), (int)head, row, v_full);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ---- MMA issue ----
-    if (lane == 0) {
-      const uint32_t idesc_s = idesc(kRows, kKeys, false), idesc_o = idesc(kRows, ls.value_dim, true);
-      const uint32_t qa = smem_u32(q_smem), ka = smem_u32(k_smem), va = smem_u32(v_smem), pa = smem_u32(p_smem);
-      auto scores = [&](uint32_t j) -> bool {
-        if (!wait(k_full, j & 1)) return false;
-        tc_fence_after();
+    const bool elected = elect_one();
+    const uint32_t idesc_s = idesc(kRows, kKeys, false), idesc_o = idesc(kRows, ls.value_dim, true);
+    const uint64_t q_desc = desc_k_sw128(smem_u32(q_smem)), k_desc = desc_k_sw128(smem_u32(k_smem)), p_desc = desc_k_sw128(smem_u32(p_smem)),
+                   v_desc = desc_mn_sw128(smem_u32(v_smem), kKSlab, 1024);
+    auto scores = [&](uint32_t j) -> bool {
+      if (!arrived(k_full, j & 1)) return false;
+      tc_fence_after();
+      if (elected) {
         const uint32_t d = tmem_base + (j & 1) * kKeys;
         uint32_t fresh = 0;
         for (uint32_t ks = 0; ks < ls.dim / 16; ++ks, fresh = 1)
-          umma_bf16(d, desc_k_sw128(qa + (ks >> 2) * kQSlab + (ks & 3) * 32), desc_k_sw128(ka + (ks >> 2) * kKSlab + (ks & 3) * 32), idesc_s, fresh);
+          umma_bf16(d, q_desc + (((ks >> 2) * kQSlab + (ks & 3) * 32) >> 4), k_desc + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s, fresh);
         for (uint32_t ks = 0; ks < ls.rot_dim / 16; ++ks, fresh = 1) {
           const uint32_t h = lay.dim_slabs + (ks >> 2);
-          umma_bf16(d, desc_k_sw128(qa + h * kQSlab + (ks & 3) * 32), desc_k_sw128(ka + h * kKSlab + (ks & 3) * 32), idesc_s, fresh);
+          umma_bf16(d, q_desc + ((h * kQSlab + (ks & 3) * 32) >> 4), k_desc + ((h * kKSlab + (ks & 3) * 32) >> 4), idesc_s, fresh);
         }
         umma_commit(&s_ready[j & 1]);
         umma_commit(k_empty);
-        return true;
-      };
-      ok = wait(q_ready, 0) && scores(0);
-      for (uint32_t j = 0; ok && j < ntiles; ++j) {
-        if (j + 1 < ntiles && !scores(j + 1)) { ok = false; break; }
-        if (!wait(p_ready, j & 1) || !wait(v_full, j & 1)) { ok = false; break; }
-        tc_fence_after();
+      }
+      __syncwarp();
+      return true;
+    };
+    ok = arrived(q_ready, 0) && scores(0);
+    for (uint32_t j = 0; ok && j < ntiles; ++j) {
+      if (j + 1 < ntiles && !scores(j + 1)) { ok = false; break; }
+      if (!arrived(p_ready, j & 1) || !arrived(v_full, j & 1)) { ok = false; break; }
+      tc_fence_after();
+      if (elected) {
 #pragma unroll
         for (uint32_t ks = 0; ks < kKeys / 16; ++ks)
-          umma_bf16(tmem_base + kTmemO, desc_k_sw128(pa + ks * 32), desc_mn_sw128(va + ks * (16 * 128), kKSlab, 1024), idesc_o,
-                    (j > 0 || ks > 0) ? 1u : 0u);
+          umma_bf16(tmem_base + kTmemO, p_desc + ks * 2, v_desc + ks * (16 * 128 >> 4), idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
         umma_commit(o_ready);
       }
+      __syncwarp();
     }
   } else {
     // ---- softmax: thread = row ----
