@@ -353,8 +353,8 @@ bool moe_tc_supported(MoeShape s) {
 int launch_moe_product_tc(const MoeProduct &p, bool swiglu, uint32_t splits, MoePlan plan, cudaStream_t stream) {
   if (swiglu && splits != 1) return set_error(ORION_ERR_INTERNAL, "the fused SwiGLU epilogue needs one k split");
   switch (plan.tile_rows) {
-    case 16: return launch_product<16, 6, 3, 1>(p, swiglu, splits, plan, stream);
-    case 32: return launch_product<32, 6, 3, 1>(p, swiglu, splits, plan, stream);
+    case 16: return launch_product<16, 4, 3, 1>(p, swiglu, splits, plan, stream);
+    case 32: return launch_product<32, 4, 2, 1>(p, swiglu, splits, plan, stream);
     case 64: return launch_product<64, 5, 3, 1>(p, swiglu, splits, plan, stream);
     case 128: return launch_product<128, 4, 2, 1>(p, swiglu, splits, plan, stream);
     default: return launch_pairs(p, swiglu, splits, plan, stream);
