@@ -90,17 +90,17 @@ struct PairConfig {
 };
 constexpr uint32_t kPairs = 74;  // of 148 SMs
 
-// A tile: weight rows w_row .. + 255 of *w against token rows x_row .. + cols - 1 of *x (cols a multiple of 16 up to 256), stages kb .. end of k.
+// A tile: weight rows w_row .. + 255 of *w against token rows x_row .. + cols - 1 of *x (cols a multiple of 32 up to 256, as a pair's MMA takes them; boxes of `box` token rows, at
+// least half of cols and a multiple of 8), stages kb .. end of k.
 struct PairJob {
   const CUtensorMap *w, *x;
-  uint32_t w_row, x_row, cols, kb, end;
+  uint32_t w_row, x_row, cols, box, kb, end;
 };
 
 // The body of a kernel of pairs (grid: two CTAs each, cluster of two). Work provides
 //   total()          tiles of the launch
 //   early(id)        whether tile `id` is known before the preceding kernel has ended
 //   job(id)          the tile, a Job; one without stages (kb == end) is passed over
-//   x_box()          token rows of a box of every x map: at least half of any tile's columns, a multiple of 8
 //   Job              what job() returns: a PairJob, and what store() needs
 //   store(j, row, c, r)  columns c .. c + 15 of weight row w_row + row (of 32 in a warp, one a lane), f32
 template <typename Work>
@@ -148,13 +148,12 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
   if (warp == 0) {
     // Producer: this CTA's weight rows and its half of the token rows; the bytes of both CTAs are counted on the leader's barrier. Weights are
     // immutable: those of the first tile are asked for before the wait for the kernel that makes the activations, where the tile is known.
-    const uint32_t box = work.x_box(), x_bytes = 2 * box * Cfg::kSlabK * 2;
     const bool elected = elect_one();
     uint32_t it = 0, early = 0;
     auto load_w = [&](uint32_t s, uint32_t kb, const PairJob &j) {
       if (!elected) return;
       const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
-      if (leader) mbar_arrive_expect_tx(&full[s], 2 * (Cfg::kWBytes + x_bytes));
+      if (leader) mbar_arrive_expect_tx(&full[s], 2 * (Cfg::kWBytes + 2 * j.box * Cfg::kSlabK * 2));
 #pragma unroll
       for (uint32_t h = 0; h < 2; ++h)
         tma_load_2d_pair(w_ring + s * Cfg::kWBytes + h * Cfg::kWSlab, j.w, (int)(kb * Cfg::kStageK + h * Cfg::kSlabK), (int)(j.w_row + rank * Cfg::kRows), bar);

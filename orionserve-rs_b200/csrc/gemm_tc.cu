@@ -360,19 +360,23 @@ struct ProjectionWork {
   struct Job : PairJob {
     float *out;
   };
-  const CUtensorMap *map_w, *map_x;
+  const CUtensorMap *map_w, *map_x, *map_tail;
   float *partial;
   bf16 *act;
   const float *bias;
-  uint32_t M, N, splits, tokn, ldc, epilogue, tiles_x, tiles_y, stages;
+  uint32_t M, N, splits, tokn, whole, tail, ldc, epilogue, tiles_x, tiles_y, stages;
 
-  __device__ __forceinline__ uint32_t total() const { return tiles_x * tiles_y * splits; }
-  __device__ __forceinline__ uint32_t x_box() const { return tokn / 2; }
+  // `whole` tiles, and those after them in `tail` pieces each
+  __device__ __forceinline__ uint32_t total() const { return whole + (tiles_x * tiles_y * splits - whole) * tail; }
   __device__ __forceinline__ bool early(uint32_t) const { return true; }
   __device__ __forceinline__ Job job(uint32_t id) const {  // the k split slowest
+    const bool piece = id >= whole;
+    const uint32_t at = piece ? (id - whole) % tail : 0, cols = piece ? tokn / tail : tokn;
+    if (piece) id = whole + (id - whole) / tail;
     const uint32_t plane = tiles_x * tiles_y, split = id / plane;
     const TileXy t = raster(id % plane, tiles_x, tiles_y);
-    return {{map_w, map_x, t.x * (2 * kTileN), t.y * tokn, tokn, (uint32_t)((uint64_t)split * stages / splits), (uint32_t)((uint64_t)(split + 1) * stages / splits)},
+    return {{map_w, piece ? map_tail : map_x, t.x * (2 * kTileN), t.y * tokn + at * cols, cols, cols / 2, (uint32_t)((uint64_t)split * stages / splits),
+             (uint32_t)((uint64_t)(split + 1) * stages / splits)},
             partial + (size_t)split * M * N};
   }
   __device__ __forceinline__ void store(const Job &j, uint32_t row, uint32_t c, uint32_t (&r)[16]) const {
@@ -410,10 +414,10 @@ struct ProjectionWork {
 
 template <int OUT>
 __global__ void __launch_bounds__(PairConfig::kThreads)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, float *__restrict__ partial,
-                 bf16 *__restrict__ act, uint32_t M, uint32_t N, uint32_t K, uint32_t splits, uint32_t tokn, uint32_t ldc, uint32_t epilogue,
-                 ReadyWait ready, const float *__restrict__ bias) {
-  const ProjectionWork<OUT> work{&map_w, &map_x, partial, act, bias, M, N, splits, tokn, ldc, epilogue, (N + 2 * kTileN - 1) / (2 * kTileN),
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_tail,
+                 float *__restrict__ partial, bf16 *__restrict__ act, uint32_t M, uint32_t N, uint32_t K, uint32_t splits, uint32_t tokn, uint32_t whole,
+                 uint32_t tail, uint32_t ldc, uint32_t epilogue, ReadyWait ready, const float *__restrict__ bias) {
+  const ProjectionWork<OUT> work{&map_w, &map_x, &map_tail, partial, act, bias, M, N, splits, tokn, whole, tail, ldc, epilogue, (N + 2 * kTileN - 1) / (2 * kTileN),
                                  (M + tokn - 1) / tokn, (K + PairConfig::kStageK - 1) / PairConfig::kStageK};
   run_pairs(work, ready, &g_gemm_error);
 }
@@ -507,26 +511,34 @@ int launch_tc(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float *p
 // all (359-399 ns with 256 tokens, 285-308 with 192, 240-255 with 128). About 3 us for the last tile's epilogue; the consumer reads every k split's
 // slab again. Against a sweep of 22 shapes of 300 to 7006 rows, every tile and 1 to 4 splits, the choice is 1.8 % off the best on average.
 uint32_t pair_tiles(uint32_t rows, uint32_t n, uint32_t tokn) { return (n + 2 * kTileN - 1) / (2 * kTileN) * ((rows + tokn - 1) / tokn); }
-uint64_t pair_cost(uint32_t rows, uint32_t n, uint32_t k, uint32_t splits, uint32_t tokn) {
+// A last round that is nearly empty costs as much as a full one: its tiles are cut into `tail` pieces of tokn / tail tokens each, so that all pairs have
+// work (512 rows of the 8B shape's gate/up: 224 tiles are three rounds and two tiles; those go as 16 pieces of 32 tokens, 101 -> 95 us).
+struct PairPlan {
+  uint32_t tokn = PairConfig::kMaxTokens, tail = 1;
+  uint64_t cost = ~0ull;
+};
+PairPlan pair_plan(uint32_t rows, uint32_t n, uint32_t k, uint32_t splits) {
   const uint64_t stages = (k + PairConfig::kStageK - 1) / PairConfig::kStageK, slabs = 2 * ((stages + splits - 1) / splits);
-  const uint64_t tiles = (uint64_t)pair_tiles(rows, n, tokn) * splits, rounds = (tiles + kPairs - 1) / kPairs;
-  const uint64_t slab = std::max<uint64_t>(tokn + 16, std::min<uint64_t>(tiles, kPairs) * (2 * kTileN + tokn) / 128);
-  return rounds * (slabs * slab + 2 * tokn) + 9 * tokn + (uint64_t)(splits - 1) * ((rows + 15) / 16 * 16) * n / 1300;
-}
-uint32_t pair_tokens(uint32_t rows, uint32_t n, uint32_t k, uint32_t splits) {
-  uint32_t best = PairConfig::kMaxTokens;
-  for (uint32_t t = best - 16; t >= 128; t -= 16)
-    if (pair_cost(rows, n, k, splits, t) < pair_cost(rows, n, k, splits, best)) best = t;
+  auto round = [&](uint64_t busy, uint32_t cols) { return slabs * std::max<uint64_t>(cols + 16, busy * (2 * kTileN + cols) / 128) + 2 * cols; };
+  PairPlan best;
+  for (uint32_t t = PairConfig::kMaxTokens; t >= 128; t -= 32) {  // a pair's MMA takes multiples of 32 columns
+    const uint64_t tiles = (uint64_t)pair_tiles(rows, n, t) * splits, rest = tiles % kPairs, full = tiles / kPairs * round(kPairs, t);
+    for (uint32_t s = 1; s <= t / 32; ++s) {
+      if (t / 32 % s || (s > 1 && (rest == 0 || rest * s > kPairs))) continue;
+      const uint64_t cost = full + (rest ? round(rest * s, t / s) : 0) + 9 * (t / s) + (uint64_t)(splits - 1) * ((rows + 15) / 16 * 16) * n / 1300;
+      if (cost < best.cost) best = {t, s, cost};
+    }
+  }
   return best;
 }
 // A k split has to gain a tenth: it keeps an activation out of the epilogue. Two full rounds and more are never split. The same for all row counts
-// of a run 16 j + 1 .. 16 (j + 1), since token tiles are multiples of 16.
+// of a run 16 j + 1 .. 16 (j + 1), since token tiles are multiples of 32.
 uint32_t pair_splits(uint32_t rows, uint32_t n, uint32_t k) {
   uint32_t best = 1;
   if (pair_tiles(rows, n, PairConfig::kMaxTokens) > 2 * kPairs) return best;
-  uint64_t cost = pair_cost(rows, n, k, 1, pair_tokens(rows, n, k, 1)) * 9 / 10;
+  uint64_t cost = pair_plan(rows, n, k, 1).cost * 9 / 10;
   for (uint32_t s = 2; s <= 4 && k / s >= 8 * kSlabK; ++s) {
-    const uint64_t c = pair_cost(rows, n, k, s, pair_tokens(rows, n, k, s));
+    const uint64_t c = pair_plan(rows, n, k, s).cost;
     if (c < cost) best = s, cost = c;
   }
   return best;
@@ -541,13 +553,15 @@ int launch_pair_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, f
   using Cfg = PairConfig;
   static bool attr_set[kMaxDeviceOrdinals] = {};
   ORION_CUDA_CHECK("gemm_pair attr", ensure_dynamic_smem(gemm_pair_kernel<OUT>, Cfg::kSmemBytes, attr_set));
-  const uint32_t tokn = pair_tokens(rows, n, k, splits);
-  const CUtensorMap *mw, *mx;
+  const PairPlan plan = pair_plan(rows, n, k, splits);
+  const uint32_t tokn = plan.tokn, tiles = pair_tiles(rows, n, tokn) * splits, whole = plan.tail > 1 ? tiles / kPairs * kPairs : tiles;
+  const CUtensorMap *mw, *mx, *mt;  // entries of a map that keeps its nodes in place
   ORION_TRY(cached_map(w, n, k, ldw, kTileN, &mw));
   ORION_TRY(cached_map(x, rows, k, ldx, tokn / 2, &mx));
-  const uint32_t tiles = pair_tiles(rows, n, tokn) * splits;
-  ORION_CUDA_CHECK("gemm_pair", launch_pdl_cluster(gemm_pair_kernel<OUT>, dim3(2 * std::min(tiles, kPairs)), dim3(Cfg::kThreads), dim3(2, 1, 1), Cfg::kSmemBytes,
-                                                   stream, *mw, *mx, partial, act, rows, n, k, splits, tokn, ldc, (uint32_t)epi, ready, bias));
+  ORION_TRY(cached_map(x, rows, k, ldx, tokn / plan.tail / 2, &mt));
+  const uint32_t jobs = whole + (tiles - whole) * plan.tail;
+  ORION_CUDA_CHECK("gemm_pair", launch_pdl_cluster(gemm_pair_kernel<OUT>, dim3(2 * std::min(jobs, kPairs)), dim3(Cfg::kThreads), dim3(2, 1, 1), Cfg::kSmemBytes,
+                                                   stream, *mw, *mx, *mt, partial, act, rows, n, k, splits, tokn, whole, plan.tail, ldc, (uint32_t)epi, ready, bias));
   count_launch();
   ORION_CUDA_CHECK("gemm_pair", cudaGetLastError());
   return ORION_OK;

@@ -214,7 +214,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
 // ---- tiles of 256 rows: persistent CTA pairs (gemm_pair.cuh) ------------------------
 // A prompt's products are bound by the tensor cores like its projections, and the tiles of the list are of unequal size: the pairs go from tile to tile,
-// entries without rows cost nothing and a tile with fewer rows takes as many columns as it has (in sixteens). Measured against one CTA per two weight
+// entries without rows cost nothing and a tile with fewer rows takes as many columns as it has (in steps of 32). Measured against one CTA per two weight
 // tiles and 256 rows, up and down: 7006 rows, width 2048, 16 experts of 1408 and a shared one of 2816: 343 + 160 -> 210 + 131 us; 2048 rows, experts
 // of 2112 without gates, a shared one of 4224: 115 + 80 -> 78 + 71.
 template <int GATED>
@@ -234,7 +234,6 @@ struct MixtureWork {
   __device__ __forceinline__ static uint32_t wide(uint32_t n) { return (n + 2 * PairConfig::kRows - 1) / (2 * PairConfig::kRows); }
   __device__ __forceinline__ uint32_t shared_total() const { return a.shared_tiles * wide(a.shared_n); }
   __device__ __forceinline__ uint32_t total() const { return shared_total() + list * wide(a.n); }
-  __device__ __forceinline__ uint32_t x_box() const { return PairConfig::kMaxTokens / 2; }
   __device__ __forceinline__ bool early(uint32_t id) const { return id < shared_total(); }
   __device__ __forceinline__ Job job(uint32_t id) const {
     constexpr uint32_t kRows = PairConfig::kMaxTokens;
@@ -247,7 +246,7 @@ struct MixtureWork {
     j.n0 = t.x * 2 * PairConfig::kRows;
     j.w = j.shared ? map_sw : map_w, j.x = j.shared ? map_sx : map_x;
     j.w_row = j.tile.expert * j.n + j.n0;  // weight rows past the matrix read as zeros, rows past the expert belong to the next one
-    j.x_row = j.tile.row, j.cols = (j.tile.count + 15) / 16 * 16;
+    j.x_row = j.tile.row, j.cols = (j.tile.count + 31) / 32 * 32, j.box = kRows / 2;
     j.kb = 0, j.end = j.tile.count > 0 ? ((j.shared ? a.shared_k : a.k) + PairConfig::kStageK - 1) / PairConfig::kStageK : 0;
     return j;
   }

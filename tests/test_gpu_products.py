@@ -12,6 +12,7 @@ SHAPES = [
     (513, 130, 136),    # one row in the last token tile
     (700, 8, 1096),     # fewer weight rows than a quarter of a warpgroup
     (1031, 6400, 136),  # more than one round of the 74 pairs, ragged
+    (512, 9728, 264),   # two tiles more than a round: the last ones in pieces
     (2065, 2432, 392),  # nine token tiles: a group of eight and one more
 ]
 
