@@ -22,10 +22,9 @@
 // tensor memory.
 #include "kernels.h"
 #include "tcgen05.cuh"
+#include "value_cache.h"
 
 #include <cstdlib>
-#include <map>
-#include <mutex>
 #include <tuple>
 
 namespace orion {
@@ -455,47 +454,39 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 
 // The K or the V rows of the arena as [chunk = (layer, block, kv head)][16 slots][dims]; a box is 16 rows x 64 dims with
 // no swizzle of its own (the rows are stored pre-permuted).
-int arena_map(const bf16 *arena, KvLayout kv, bool values, const CUtensorMap **out) {
-  static std::mutex mu;
-  static std::map<std::tuple<const void *, uint64_t, uint32_t, uint64_t, bool>, CUtensorMap> cache;
+int arena_map(const bf16 *arena, KvLayout kv, bool values, CUtensorMap *out) {
+  static ValueCache<std::tuple<const void *, uint64_t, uint32_t, uint64_t, bool>, CUtensorMap> cache(4096);
   EncodeFn fn = encode_fn();
   if (!fn) return set_error(ORION_ERR_BACKEND, "backend cuda failed at tensor map: driver entry point missing");
   const uint64_t chunks = (uint64_t)kv.num_layers * kv.num_blocks * kv.num_kv_heads;
-  std::lock_guard<std::mutex> lock(mu);
-  auto key = std::make_tuple((const void *)arena, chunks, kv.head_dim, (uint64_t)kv.chunk_elems(), values);
-  auto it = cache.find(key);
-  if (it == cache.end()) {
-    if (cache.size() > 4096) cache.clear();
-    CUtensorMap m;
+  return cache.get({arena, chunks, kv.head_dim, (uint64_t)kv.chunk_elems(), values}, out, [&](CUtensorMap *m) -> int {
     const cuuint64_t cols = values ? kv.v_dim() : kv.head_dim;
     const cuuint64_t dims[3] = {cols, (cuuint64_t)kBlk, chunks};
     const cuuint64_t strides[2] = {cols * 2, (cuuint64_t)kv.chunk_elems() * 2};
     bf16 *base = const_cast<bf16 *>(arena) + (values && !kv.factor_elems ? (size_t)kBlk * kv.head_dim : 0);
     const cuuint32_t box[3] = {64, (cuuint32_t)kBlk, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, estr,
+    const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
       return set_error(ORION_ERR_BACKEND, "backend cuda failed at tensor map: encode returned %d (arena of %llu chunks)", (int)r,
                        (unsigned long long)chunks);
-    it = cache.emplace(key, m).first;
-  }
-  *out = &it->second;
-  return ORION_OK;
+    return ORION_OK;
+  });
 }
 
 template <int DK, int DV, int FORM>
 int launch_prefill_tc(const bf16 *q, const bf16 *arena, KvLayout kv, uint32_t layer, AttnBatch batch, const PrefillTile *tiles,
                       uint32_t num_tiles, uint32_t q_heads, AttnForm form, bf16 *out, cudaStream_t stream) {
   using Cfg = PrefillTcConfig<DK, DV, FORM == 3>;
-  const CUtensorMap *mk = nullptr, *mv = nullptr;
+  CUtensorMap mk, mv;
   ORION_TRY(arena_map(arena, kv, false, &mk));
   ORION_TRY(arena_map(arena, kv, true, &mv));
   static bool attr_set[kMaxDeviceOrdinals] = {};
   ORION_CUDA_CHECK("paged_prefill_tc attr", ensure_dynamic_smem(paged_prefill_tc_kernel<DK, DV, FORM>, Cfg::kSmem, attr_set));
   ORION_CUDA_CHECK("paged_prefill_tc", launch_pdl(paged_prefill_tc_kernel<DK, DV, FORM>, dim3(kv.num_kv_heads, num_tiles), dim3(kThreads),
-                                                  (size_t)Cfg::kSmem, stream, *mk, *mv, q, arena, kv, layer, batch, tiles, q_heads, out, form));
+                                                  (size_t)Cfg::kSmem, stream, mk, mv, q, arena, kv, layer, batch, tiles, q_heads, out, form));
   count_launch();
   ORION_CUDA_CHECK("paged_prefill_tc", cudaGetLastError());
   return ORION_OK;

@@ -25,11 +25,10 @@
 // Every wait is bounded; a wait that runs out sets a device error word and the
 // CTA still releases its tensor memory before returning.
 #include "gemm_pair.cuh"
+#include "value_cache.h"
 
 #include <algorithm>
 #include <cstdlib>
-#include <map>
-#include <mutex>
 #include <tuple>
 
 namespace orion {
@@ -442,30 +441,9 @@ int make_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k, uint
   return ORION_OK;
 }
 
-struct MapKey {
-  const void *base;
-  uint64_t rows, k, ld;
-  uint32_t box_rows;
-  bool operator<(const MapKey &o) const {
-    return std::tie(base, rows, k, ld, box_rows) < std::tie(o.base, o.rows, o.k, o.ld, o.box_rows);
-  }
-};
-
-int cached_map(const void *base, uint64_t rows, uint64_t k, uint64_t ld, uint32_t box_rows,
-               const CUtensorMap **out) {
-  static std::mutex mu;
-  static std::map<MapKey, CUtensorMap> cache;
-  std::lock_guard<std::mutex> lock(mu);
-  MapKey key{base, rows, k, ld, box_rows};
-  auto it = cache.find(key);
-  if (it == cache.end()) {
-    if (cache.size() > 65536) cache.clear();
-    CUtensorMap m;
-    ORION_TRY(make_map(&m, base, rows, k, ld, box_rows));
-    it = cache.emplace(key, m).first;
-  }
-  *out = &it->second;
-  return ORION_OK;
+int cached_map(const void *base, uint64_t rows, uint64_t k, uint64_t ld, uint32_t box_rows, CUtensorMap *out) {
+  static ValueCache<std::tuple<const void *, uint64_t, uint64_t, uint64_t, uint32_t>, CUtensorMap> cache(65536);
+  return cache.get({base, rows, k, ld, box_rows}, out, [&](CUtensorMap *m) { return make_map(m, base, rows, k, ld, box_rows); });
 }
 
 template <bool ACT, int TOKN, int WST, int XST, int MT>
@@ -480,17 +458,17 @@ int launch_tc_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, flo
   if (MT > 1 && cluster_reduce) return set_error(ORION_ERR_INTERNAL, "cluster split-K is built for one weight tile per CTA");
   static bool attr_set[kMaxDeviceOrdinals] = {};
   ORION_CUDA_CHECK("gemm_tc attr", ensure_dynamic_smem(gemm_tc_kernel<TOKN, WST, XST, MT, ACT>, Cfg::kSmemBytes, attr_set));
-  const CUtensorMap *mw, *mx;
+  CUtensorMap mw, mx;
   ORION_TRY(cached_map(w, n, k, ldw, kTileN, &mw));
   ORION_TRY(cached_map(x, rows, k, ldx, TOKN, &mx));
   dim3 grid((n + MT * kTileN - 1) / (MT * kTileN), (rows + TOKN - 1) / TOKN, splits);
   if (cluster_reduce)
     ORION_CUDA_CHECK("gemm_tc", launch_pdl_cluster(gemm_tc_kernel<TOKN, WST, XST, MT, ACT>, grid, dim3(kThreads), dim3(1, 1, splits),
-                                                   Cfg::kSmemBytes, stream, *mw, *mx, partial, act, rows, n, k, splits,
+                                                   Cfg::kSmemBytes, stream, mw, mx, partial, act, rows, n, k, splits,
                                                    1u, ldc, (uint32_t)epi, ready, bias));
   else
     ORION_CUDA_CHECK("gemm_tc", launch_pdl(gemm_tc_kernel<TOKN, WST, XST, MT, ACT>, grid, dim3(kThreads), Cfg::kSmemBytes, stream,
-                                           *mw, *mx, partial, act, rows, n, k, splits, 0u, ldc, (uint32_t)epi, ready, bias));
+                                           mw, mx, partial, act, rows, n, k, splits, 0u, ldc, (uint32_t)epi, ready, bias));
   count_launch();
   ORION_CUDA_CHECK("gemm_tc", cudaGetLastError());
   return ORION_OK;
@@ -555,13 +533,14 @@ int launch_pair_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, f
   ORION_CUDA_CHECK("gemm_pair attr", ensure_dynamic_smem(gemm_pair_kernel<OUT>, Cfg::kSmemBytes, attr_set));
   const PairPlan plan = pair_plan(rows, n, k, splits);
   const uint32_t tokn = plan.tokn, tiles = pair_tiles(rows, n, tokn) * splits, whole = plan.tail > 1 ? tiles / kPairs * kPairs : tiles;
-  const CUtensorMap *mw, *mx, *mt;  // entries of a map that keeps its nodes in place
+  CUtensorMap mw, mx, mt;
   ORION_TRY(cached_map(w, n, k, ldw, kTileN, &mw));
   ORION_TRY(cached_map(x, rows, k, ldx, tokn / 2, &mx));
-  ORION_TRY(cached_map(x, rows, k, ldx, tokn / plan.tail / 2, &mt));
+  mt = mx;
+  if (plan.tail > 1) ORION_TRY(cached_map(x, rows, k, ldx, tokn / plan.tail / 2, &mt));
   const uint32_t jobs = whole + (tiles - whole) * plan.tail;
   ORION_CUDA_CHECK("gemm_pair", launch_pdl_cluster(gemm_pair_kernel<OUT>, dim3(2 * std::min(jobs, kPairs)), dim3(Cfg::kThreads), dim3(2, 1, 1), Cfg::kSmemBytes,
-                                                   stream, *mw, *mx, *mt, partial, act, rows, n, k, splits, tokn, whole, plan.tail, ldc, (uint32_t)epi, ready, bias));
+                                                   stream, mw, mx, mt, partial, act, rows, n, k, splits, tokn, whole, plan.tail, ldc, (uint32_t)epi, ready, bias));
   count_launch();
   ORION_CUDA_CHECK("gemm_pair", cudaGetLastError());
   return ORION_OK;

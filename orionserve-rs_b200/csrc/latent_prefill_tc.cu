@@ -14,10 +14,9 @@
 // Every wait is bounded; a wait that runs out sets the device error word and the CTA still frees its tensor memory.
 #include "kernels.h"
 #include "tcgen05.cuh"
+#include "value_cache.h"
 
 #include <algorithm>
-#include <map>
-#include <mutex>
 #include <tuple>
 
 namespace orion {
@@ -304,30 +303,22 @@ latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
 // ---- host side -----------------------------------------------------------------
 
 // [rows][heads][cols] bf16 with `row_ld` elements between rows (heads = 1: a plain matrix); box of 64 columns x 64 rows.
-int slab_map(const bf16 *base, uint32_t cols, uint32_t heads, uint32_t rows, uint32_t row_ld, bool by_head, const CUtensorMap **out) {
-  static std::mutex mu;
-  static std::map<std::tuple<const void *, uint32_t, uint32_t, uint32_t, uint32_t, bool>, CUtensorMap> cache;
+int slab_map(const bf16 *base, uint32_t cols, uint32_t heads, uint32_t rows, uint32_t row_ld, bool by_head, CUtensorMap *out) {
+  static ValueCache<std::tuple<const void *, uint32_t, uint32_t, uint32_t, uint32_t, bool>, CUtensorMap> cache(4096);
   EncodeFn fn = encode_fn();
   if (!fn) return set_error(ORION_ERR_BACKEND, "backend cuda failed at tensor map: driver entry point missing");
-  std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_tuple((const void *)base, cols, heads, rows, row_ld, by_head);
-  auto it = cache.find(key);
-  if (it == cache.end()) {
-    if (cache.size() > 4096) cache.clear();
-    CUtensorMap m;
+  return cache.get({base, cols, heads, rows, row_ld, by_head}, out, [&](CUtensorMap *m) -> int {
     const cuuint64_t dims3[3] = {cols, heads, rows}, dims2[2] = {cols, rows};
     const cuuint64_t strides3[2] = {(cuuint64_t)cols * 2, (cuuint64_t)row_ld * 2}, strides2[1] = {(cuuint64_t)row_ld * 2};
     const cuuint32_t box3[3] = {64, 1, kKeys}, box2[2] = {64, kKeys}, ones[3] = {1, 1, 1};
-    const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, by_head ? 3 : 2, const_cast<bf16 *>(base), by_head ? dims3 : dims2,
+    const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, by_head ? 3 : 2, const_cast<bf16 *>(base), by_head ? dims3 : dims2,
                           by_head ? strides3 : strides2, by_head ? box3 : box2, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
       return set_error(ORION_ERR_BACKEND, "backend cuda failed at tensor map: encode returned %d (%u columns, %u heads, %u rows)", (int)r,
                        cols, heads, rows);
-    it = cache.emplace(key, m).first;
-  }
-  *out = &it->second;
-  return ORION_OK;
+    return ORION_OK;
+  });
 }
 
 }  // namespace
@@ -352,7 +343,7 @@ int launch_latent_prefill(const bf16 *q, const bf16 *expanded, const bf16 *rotat
                           uint32_t ldo, cudaStream_t stream) {
   if (num_tiles == 0) return ORION_OK;
   if (!latent_prefill_supported(ls)) return set_error(ORION_ERR_INTERNAL, "tensor-core latent attention does not cover this shape");
-  const CUtensorMap *mk = nullptr, *mr = nullptr, *mv = nullptr;
+  CUtensorMap mk, mr, mv;
   const uint32_t ld = ls.heads * (ls.dim + ls.value_dim);
   ORION_TRY(slab_map(expanded, ls.dim, ls.heads, rows_capacity, ld, true, &mk));
   ORION_TRY(slab_map(expanded + ls.heads * ls.dim, ls.value_dim, ls.heads, rows_capacity, ld, true, &mv));
@@ -363,8 +354,8 @@ int launch_latent_prefill(const bf16 *q, const bf16 *expanded, const bf16 *rotat
   const uint32_t smem = std::max(PrefillSmem(ls).total, tmem_columns(ls.value_dim) == 256 ? 77u * 1024 : 132u * 1024);
   static bool attr_set[kMaxDeviceOrdinals] = {};
   ORION_CUDA_CHECK("latent_prefill attr", ensure_dynamic_smem(latent_prefill_tc_kernel, 226 * 1024, attr_set));
-  ORION_CUDA_CHECK("latent_prefill", launch_pdl(latent_prefill_tc_kernel, dim3(ls.heads, num_tiles), dim3(kThreads), smem, stream, *mk, *mr,
-                                                *mv, q, gate_partial, splits, split_stride, tiles, ls, out, ldo));
+  ORION_CUDA_CHECK("latent_prefill", launch_pdl(latent_prefill_tc_kernel, dim3(ls.heads, num_tiles), dim3(kThreads), smem, stream, mk, mr,
+                                                mv, q, gate_partial, splits, split_stride, tiles, ls, out, ldo));
   count_launch();
   ORION_CUDA_CHECK("latent_prefill", cudaGetLastError());
   return ORION_OK;

@@ -11,10 +11,9 @@
 //              an activation f(w u) without a gate
 // Every wait is bounded; a wait that runs out sets the device error word and the CTA still frees its tensor memory.
 #include "gemm_pair.cuh"
+#include "value_cache.h"
 
 #include <algorithm>
-#include <map>
-#include <mutex>
 #include <tuple>
 
 namespace orion {
@@ -263,27 +262,20 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 }
 
 // [rows][k] bf16, box of 64 k x box_rows, 128-byte swizzle.
-int matrix_map(const bf16 *base, uint64_t rows, uint64_t k, uint32_t box_rows, const CUtensorMap **out) {
-  static std::mutex mu;
-  static std::map<std::tuple<const void *, uint64_t, uint64_t, uint32_t>, CUtensorMap> cache;
+int matrix_map(const bf16 *base, uint64_t rows, uint64_t k, uint32_t box_rows, CUtensorMap *out) {
+  static ValueCache<std::tuple<const void *, uint64_t, uint64_t, uint32_t>, CUtensorMap> cache(65536);
   EncodeFn fn = encode_fn();
   if (!fn) return set_error(ORION_ERR_BACKEND, "backend cuda failed at tensor map: driver entry point missing");
-  std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_tuple((const void *)base, rows, k, box_rows);
-  auto it = cache.find(key);
-  if (it == cache.end()) {
-    CUtensorMap m;
+  return cache.get({base, rows, k, box_rows}, out, [&](CUtensorMap *m) -> int {
     const cuuint64_t dims[2] = {k, rows}, strides[1] = {k * 2};
     const cuuint32_t box[2] = {kSlabK, box_rows}, ones[2] = {1, 1};
-    const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16 *>(base), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16 *>(base), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
       return set_error(ORION_ERR_BACKEND, "backend cuda failed at tensor map: encode returned %d (rows %llu k %llu)", (int)r, (unsigned long long)rows,
                        (unsigned long long)k);
-    it = cache.emplace(key, m).first;
-  }
-  *out = &it->second;
-  return ORION_OK;
+    return ORION_OK;
+  });
 }
 
 int product_form(const MoeProduct &p, bool gated) {
@@ -293,7 +285,7 @@ int product_form(const MoeProduct &p, bool gated) {
 template <int TOKN, int WST, int XST, int MT>
 int launch_product(const MoeProduct &p, bool swiglu, uint32_t splits, MoePlan plan, cudaStream_t stream) {
   using Cfg = MoeConfig<TOKN, WST, XST, MT>;
-  const CUtensorMap *mw, *mx, *msw, *msx;
+  CUtensorMap mw, mx, msw, msx;
   ORION_TRY(matrix_map(p.w, (uint64_t)p.experts * p.n, p.k, kTileN, &mw));
   ORION_TRY(matrix_map(p.x, p.sorted_rows, p.k, TOKN, &mx));
   msw = mw, msx = mx;
@@ -311,7 +303,7 @@ int launch_product(const MoeProduct &p, bool swiglu, uint32_t splits, MoePlan pl
                 : form == 2 ? moe_gemm_tc_kernel<TOKN, WST, XST, MT, 2>
                             : moe_gemm_tc_kernel<TOKN, WST, XST, MT, 3>;
   ORION_CUDA_CHECK("moe_gemm attr", ensure_dynamic_smem(kernel, Cfg::kSmemBytes, attr_set[form]));
-  ORION_CUDA_CHECK("moe_gemm", launch_pdl(kernel, grid, dim3(kThreads), (size_t)Cfg::kSmemBytes, stream, *mw, *mx, *msw, *msx, a));
+  ORION_CUDA_CHECK("moe_gemm", launch_pdl(kernel, grid, dim3(kThreads), (size_t)Cfg::kSmemBytes, stream, mw, mx, msw, msx, a));
   count_launch();
   ORION_CUDA_CHECK("moe_gemm", cudaGetLastError());
   return ORION_OK;
@@ -320,7 +312,7 @@ int launch_product(const MoeProduct &p, bool swiglu, uint32_t splits, MoePlan pl
 int launch_pairs(const MoeProduct &p, bool gated, uint32_t splits, MoePlan plan, cudaStream_t stream) {
   constexpr uint32_t kRows = PairConfig::kMaxTokens, kWide = 2 * PairConfig::kRows;
   if (plan.tile_rows != kRows || splits != 1) return set_error(ORION_ERR_INTERNAL, "pairs take tiles of 256 rows and one k split");
-  const CUtensorMap *mw, *mx, *msw, *msx;
+  CUtensorMap mw, mx, msw, msx;
   ORION_TRY(matrix_map(p.w, (uint64_t)p.experts * p.n, p.k, PairConfig::kRows, &mw));
   ORION_TRY(matrix_map(p.x, p.sorted_rows, p.k, kRows / 2, &mx));
   msw = mw, msx = mx;
@@ -336,7 +328,7 @@ int launch_pairs(const MoeProduct &p, bool gated, uint32_t splits, MoePlan plan,
   auto kernel = form == 0 ? moe_pair_kernel<0> : form == 1 ? moe_pair_kernel<1> : form == 2 ? moe_pair_kernel<2> : moe_pair_kernel<3>;
   ORION_CUDA_CHECK("moe_pair attr", ensure_dynamic_smem(kernel, PairConfig::kSmemBytes, attr_set[form]));
   ORION_CUDA_CHECK("moe_pair", launch_pdl_cluster(kernel, dim3(2 * std::min(total, kPairs)), dim3(PairConfig::kThreads), dim3(2, 1, 1),
-                                                  (size_t)PairConfig::kSmemBytes, stream, *mw, *mx, *msw, *msx, a, plan.tiles));
+                                                  (size_t)PairConfig::kSmemBytes, stream, mw, mx, msw, msx, a, plan.tiles));
   count_launch();
   ORION_CUDA_CHECK("moe_pair", cudaGetLastError());
   return ORION_OK;
