@@ -12,6 +12,7 @@
 #include <tuple>
 #include <vector>
 
+#include "error_words.h"
 #include "model.h"
 
 namespace orion {
@@ -598,7 +599,7 @@ int StepModel<T>::forward(const BatchView &b, float *logits_out, uint64_t logits
   }
   // The words of all translation units came with the step: only a wait that ran out (in whichever model) is looked into. The f32 build has none of
   // its own, and polls what its collectives have.
-  if (!DTypeOf<T>::is_bf16 || *h_error_ != 0) ORION_TRY(poll_errors());
+  if (poll_after_step(DTypeOf<T>::is_bf16, *h_error_)) ORION_TRY(poll_errors());
   step_done(b);
   return ORION_OK;
 }
