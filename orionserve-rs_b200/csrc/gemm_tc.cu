@@ -512,8 +512,12 @@ PairPlan pair_plan(uint32_t rows, uint32_t n, uint32_t k, uint32_t splits) {
 // A k split has to gain a tenth: it keeps an activation out of the epilogue. Two full rounds and more are never split. The same for all row counts
 // of a run 16 j + 1 .. 16 (j + 1), since token tiles are multiples of 32.
 uint32_t pair_splits(uint32_t rows, uint32_t n, uint32_t k) {
+  const uint32_t tiles = pair_tiles(rows, n, PairConfig::kMaxTokens);
   uint32_t best = 1;
-  if (pair_tiles(rows, n, PairConfig::kMaxTokens) > 2 * kPairs) return best;
+  if (tiles > 2 * kPairs) return best;
+  // One weight tile is mostly latency, and slabs of so few columns cost little: up to four splits of 512 k and more while half of the pairs are
+  // enough for them. k 2048, 16 rows of weights and the norm that reads the result: 1280 tokens 10.7 -> 9.8 us, 2048 tokens 13.5 -> 11.1.
+  if (n <= (uint32_t)kTileN) return std::max(1u, std::min({4u, k / (8 * kSlabK), kPairs / 2 / tiles}));
   uint64_t cost = pair_plan(rows, n, k, 1).cost * 9 / 10;
   for (uint32_t s = 2; s <= 4 && k / s >= 8 * kSlabK; ++s) {
     const uint64_t c = pair_plan(rows, n, k, s).cost;
@@ -555,8 +559,14 @@ int launch_pair(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float 
 // Who takes the persistent pairs: 1 (default) = batches of more than 256 rows, 2 = of more than 128 (the parity tests run this), 0 = nobody.
 // ORION_GEMM_PAIR overrides. The four projections of the 8B shape at 512 / 2048 / 8192 rows, f32 out: 188 / 611 / 2380 us with pairs, 239 / 775 / 2540
 // with one CTA per 256-token tile. At 129 to 256 rows the two are equal: the wider gate/up 3-6 % slower with pairs, the others 5-13 % faster.
+// Matrices of one weight tile (routers) are the exception: the second CTA of a pair has nothing but padding, and with more than kRouterRows tokens single
+// CTAs are faster. 16 rows of k 2048 and the norm that reads the result, 2048 / 3000 / 4096 / 8192 tokens: single CTAs 12.0 / 12.6 / 13.6 / 19.5 us, pairs
+// with the best k splits 11.1 / 12.8 / 15.3 / 23.1; 64 rows of k 4096: 14.7 / 15.4 / 16.3 / 21.4 and 12.2 / 14.6 / 17.3 / 25.3.
 int g_gemm_pair = std::getenv("ORION_GEMM_PAIR") ? std::atoi(std::getenv("ORION_GEMM_PAIR")) : 1;
-bool takes_pairs(uint32_t rows) { return g_gemm_pair >= 1 && rows > (g_gemm_pair >= 2 ? 128u : 256u); }
+constexpr uint32_t kRouterRows = 3072;
+bool takes_pairs(uint32_t rows, uint32_t n) {
+  return g_gemm_pair >= 1 && rows > (g_gemm_pair >= 2 ? 128u : 256u) && (n > (uint32_t)kTileN || rows <= kRouterRows);
+}
 
 // Tuning A/B: ORION_GEMM_PREFILL_TILES=1 keeps one weight tile per CTA for prefill-sized batches
 // (two tiles measured 3 % faster on the continuous-batching workload, gate/up only: the other
@@ -618,7 +628,7 @@ int launch_gemm_tc(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, flo
   uint32_t tt = token_tile(rows);
   // prefill batches whose 256-token tiles would leave SMs idle take 128-token tiles instead
   if (rows > 256 && g_prefill_fill == 1 && ((n + kTileN - 1) / kTileN) * ((rows + 255) / 256) < 148) tt = 128;
-  if (takes_pairs(rows) && !cluster_reduce) {
+  if (takes_pairs(rows, n) && !cluster_reduce) {
     if (splits > (k + PairConfig::kStageK - 1) / PairConfig::kStageK) return set_error(ORION_ERR_INTERNAL, "gemm split count %u leaves a split empty", splits);
     return launch_pair(x, ldx, w, ldw, partial, act, rows, n, k, splits, ldc, epi, stream, ready, bias);
   }
@@ -704,7 +714,7 @@ GemmPlan gemm_plan(bool is_bf16, uint32_t rows, uint32_t n, uint32_t k, uint32_t
         encode_fn() != nullptr))
     return p;
   p.tensor_core = true;
-  if (takes_pairs(rows)) {
+  if (takes_pairs(rows, n)) {
     p.splits = p.out_slabs = pair_splits(rows, n, k);
     return p;
   }
@@ -743,7 +753,7 @@ GemmPlan gemm_plan(bool is_bf16, uint32_t rows, uint32_t n, uint32_t k, uint32_t
 size_t gemm_partial_floats(bool is_bf16, uint32_t max_rows, uint32_t n, uint32_t k) {
   size_t best = (size_t)max_rows * n;
   if (!is_bf16) return best;
-  for (uint32_t r = 1; r <= max_rows; r = takes_pairs(r) && r < max_rows ? std::min(max_rows, (r / 16 + 1) * 16) : r + 1) {  // as in pair_splits
+  for (uint32_t r = 1; r <= max_rows; r = takes_pairs(r, n) && r < max_rows ? std::min(max_rows, (r / 16 + 1) * 16) : r + 1) {  // as in pair_splits
     const GemmPlan p = gemm_plan(true, r, n, k, k, k);
     const size_t need = (size_t)p.splits * r * n;
     if (need > best) best = need;

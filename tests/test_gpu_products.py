@@ -1,4 +1,6 @@
 """Products at the edges of their tiles: the persistent CTA pairs of more than 256 rows (tiles, k remainders, k splits, rounds), the f32 decode kernel."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -11,6 +13,11 @@ SHAPES = [
     (512, 1024, 4096),  # k splits
     (513, 130, 136),    # one row in the last token tile
     (700, 8, 1096),     # fewer weight rows than a quarter of a warpgroup
+    (2065, 18, 2048),   # one weight tile: a router's columns, k splits
+    (3072, 16, 1032),   # the most tokens of one weight tile that pairs take
+    (3073, 18, 1032),   # ... and single CTAs from there on
+    (300, 128, 72),
+    (300, 129, 72),
     (1031, 6400, 136),  # more than one round of the 74 pairs, ragged
     (512, 9728, 264),   # two tiles more than a round: the last ones in pieces
     (2065, 2432, 392),  # nine token tiles: a group of eight and one more
@@ -33,6 +40,14 @@ def test_products_of_many_rows(pkg, backend, rows, n, k):
     # and a k split one rounding more
     bound = (k / 16 + 8) * 2.0 ** -23 * size
     assert np.all(np.abs(got - exact) <= bound), float(np.max(np.abs(got - exact) / bound))
+
+
+@pytest.mark.parametrize("rows,n,k,splits", [(300, 64, 512, 1), (1280, 16, 2048, 4), (2048, 18, 2048, 4), (3072, 16, 2048, 3), (3073, 16, 2048, 4), (8192, 128, 1024, 2)])
+def test_one_weight_tile_is_split_along_k(pkg, backend, rows, n, k, splits):
+    """Routers: a single weight tile, so k splits are what fills the chip, whatever the number of tokens."""
+    ms, used = ctypes.c_float(), ctypes.c_uint32()
+    pkg.errors.check(pkg._ffi.lib().orion_cuda_linear_bench(backend._h, rows, k, n, 1, 1, ctypes.byref(ms), ctypes.byref(used)))
+    assert used.value == splits
 
 
 @pytest.mark.parametrize("rows", [1, 7, 8, 9, 64, 65])
