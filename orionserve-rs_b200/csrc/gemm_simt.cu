@@ -148,8 +148,12 @@ int launch_gemm_simt(const T *x, uint32_t ldx, const T *w, uint32_t ldw, float *
                      uint32_t n, uint32_t k, cudaStream_t stream) {
   if (rows == 0 || n == 0) return ORION_OK;
   if constexpr (sizeof(T) == 4) {
-    // Decode batches. With more rows the 4 x 4 outputs of a thread above need a quarter of the shared-memory reads.
-    if (rows <= 64 && k % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
+    // Decode batches. The 4 x 4 outputs of a thread above need a quarter of the shared-memory reads, so that kernel wins where it fills the chip: with more
+    // than 32 rows against many outputs (the head of a large vocabulary). Few / tile, us, with k 256: 16384 outputs and 64 rows 55 / 61; 28000 outputs
+    // 59 / 65 with 40 rows, 70 / 66 with 48, 92 / 69 with 64; 128256 outputs 209 / 233 with 32 rows, 259 / 235 with 40, 411 / 240 with 64; k 4096, 14336
+    // outputs and 64 rows 716 / 1152.
+    const bool few_rows = rows <= 32 || (rows <= 64 && (uint64_t)((rows + 7) / 8 * 8) * n < 1300000);
+    if (few_rows && k % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
       const dim3 few((n + kFewCols - 1) / kFewCols, (rows + kFewRows - 1) / kFewRows);
       ORION_CUDA_CHECK("gemm_simt", launch_pdl(gemm_simt_few_kernel, few, dim3(kFewRows * kFewCols), 0, stream, x, ldx, w, ldw, out, rows, n, k));
       count_launch();

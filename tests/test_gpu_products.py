@@ -58,3 +58,12 @@ def test_f32_products_of_few_rows_are_bit_exact(pkg, backend, rows, n, k):
     rng = np.random.default_rng(rows * 7 + n + k)
     x, w = rng.standard_normal((rows, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
     assert np.array_equal(pkg.ops.linear(backend, x, w), oracle.linear(x, w))
+
+
+@pytest.mark.parametrize("rows,n", [(32, 40001), (33, 32499), (33, 32500), (57, 20312), (64, 20313), (65, 400)])
+def test_f32_products_on_both_sides_of_the_rule_are_bit_exact(pkg, backend, rows, n):
+    """More than 32 rows against a large vocabulary go to the tiles of 64 x 64 outputs."""
+    from oracle import binding as oracle
+    rng = np.random.default_rng(rows + n)
+    x, w = rng.standard_normal((rows, 20)).astype(np.float32), rng.standard_normal((n, 20)).astype(np.float32)
+    assert np.array_equal(pkg.ops.linear(backend, x, w), oracle.linear(x, w))
