@@ -577,6 +577,7 @@ struct MoePlan {
   uint32_t tiles;                 // entries of the tile list
   uint32_t up_splits, down_splits;  // k splits of the two products
   bool tensor_core;
+  uint32_t live = 0;  // batches of up to 32 rows: about how many of the tiles have rows
 };
 MoePlan moe_plan(bool is_bf16, MoeShape s, uint32_t rows);
 constexpr uint32_t kMoeMaxExperts = 1024;

@@ -11,6 +11,7 @@
 #include "mma.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace orion {
 namespace {
@@ -409,8 +410,11 @@ MoePlan moe_plan(bool is_bf16, MoeShape s, uint32_t rows) {
   }
   const uint64_t busy = std::min<uint64_t>(s.experts, choices);  // experts that have rows, at most
   p.tiles = (uint32_t)(busy + choices / p.tile_rows);
+  // As many as fall to different experts if all are as likely, and one more: too few rounds of CTAs cost more than too many.
+  if (rows <= 32) p.live = (uint32_t)std::min((double)busy, s.experts * (1.0 - std::pow(1.0 - (double)s.top / s.outputs(), rows)) + 1.0);
   if (p.tensor_core && rows <= 64) {
-    // k splits until a wave of two CTAs per SM is full, at least four k slabs each
+    // k splits until a wave of two CTAs per SM is full, at least four k slabs each. (Three share an SM only where a product has more tiles than that,
+    // see launch_moe_product_tc.)
     auto splits = [&](uint32_t n, uint32_t shared_n, uint32_t k) {
       const uint64_t ctas = busy * ((n + 127) / 128) + (shared_n + 127) / 128;
       const uint32_t most = std::max(1u, (k + 63) / 64 / 4);
