@@ -76,13 +76,15 @@ embed_rmsnorm_kernel(const T *__restrict__ embed, const uint32_t *__restrict__ t
 }
 
 // Row-wise kernels of 128-bit loads keep CHUNKS float4 groups of a row per thread in registers. Few rows: as many threads as groups (up to 1024), so
-// that a row is one round trip to memory. More rows than such CTAs fit on the chip at once (two per SM): a quarter of the threads with four groups
-// each, so that an SM holds more rows and has more loads in flight. Figures at the kernels.
+// that a row is one round trip to memory. More rows than such CTAs of 1024 threads fit on the chip at once (two per SM): a quarter of the threads with
+// four groups each, so that an SM holds more rows and has more loads in flight. Figures at the kernels. Sums of several slabs have their loads in flight
+// anyway, and stay as they are while the smaller CTAs of shorter rows all fit: 297 rows of 1024, three slabs 2.8 us, 3.8 with a quarter of the
+// threads; 400 rows of 2048, four slabs 4.1, 4.8; 1024 rows of 2048, four slabs 7.8, 5.9.
 constexpr uint32_t kManyRows = 2 * 148;
-inline uint32_t row_threads(uint32_t nvec, uint32_t rows) {
+inline uint32_t row_threads(uint32_t nvec, uint32_t rows, uint32_t slabs) {
   constexpr uint32_t most = 1024;
   const uint32_t one = nvec >= most ? most : (nvec + 31) / 32 * 32;
-  if (rows <= kManyRows) return one;
+  if (rows <= kManyRows || (slabs > 1 && rows <= kManyRows * (most / one))) return one;
   const uint32_t four = ((nvec + 3) / 4 + 31) / 32 * 32;
   return four < 128 ? (one < 128 ? one : 128) : (four > most ? most : four);
 }
@@ -601,7 +603,7 @@ int launch_embed_rmsnorm(const T *embed, const uint32_t *tokens, const float *no
                          cudaStream_t stream, float scale, const float *shift) {
   if (rows == 0) return ORION_OK;
   if (hidden_size % 4 == 0 && hidden_size / 4 <= 4096) {
-    const uint32_t nvec = hidden_size / 4, threads = row_threads(nvec, rows), chunks = (nvec + threads - 1) / threads;
+    const uint32_t nvec = hidden_size / 4, threads = row_threads(nvec, rows, 1), chunks = (nvec + threads - 1) / threads;
     auto kernel = chunks == 1 ? embed_rmsnorm_vec_kernel<T, 1> : chunks == 2 ? embed_rmsnorm_vec_kernel<T, 2> : embed_rmsnorm_vec_kernel<T, 4>;
     ORION_CUDA_CHECK("embed_rmsnorm", launch_pdl(kernel, dim3(rows), dim3(threads), 0, stream, embed, tokens, norm_w, eps, hidden, normed, hidden_size,
                                                  scale, shift));
@@ -713,7 +715,7 @@ int launch_residual_rmsnorm(const float *partial, uint32_t splits, size_t split_
                             cudaStream_t stream, uint32_t *ready) {
   if (out_rows == 0) return ORION_OK;
   if (hidden_size % 4 == 0 && hidden_size / 4 <= 4096 && split_stride % 4 == 0) {
-    const uint32_t nvec = hidden_size / 4, threads = row_threads(nvec, out_rows);
+    const uint32_t nvec = hidden_size / 4, threads = row_threads(nvec, out_rows, splits);
     const uint32_t chunks = (nvec + threads - 1) / threads;
     if (chunks == 1)
       return launch_residual_vec<T, 1>(partial, splits, split_stride, hidden, norm_w, eps, out, row_map,
