@@ -78,10 +78,17 @@ __device__ __forceinline__ void store_chunk(const TcArgs &a, bool shared, const 
         if (c + 2 * jj + odd < tile.count) *to = v[jj];
     }
   } else if (nn < n) {
-    float *out = shared ? a.shared_out + (size_t)split * a.rows * n : a.out + (size_t)split * a.sorted_rows * n;
+    // One addition per store: with an address and a test worked out for each, these stores took longer than the main loop of a short k (the last example
+    // below: 114 us instead of 72).
+    float *out = shared ? a.shared_out + (size_t)split * a.rows * n : a.out + (size_t)split * a.sorted_rows * n, *to = out + (size_t)(tile.row + c) * n + nn;
+    if (c + 16 <= tile.count) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (c + j < tile.count) out[(size_t)(tile.row + c + j) * n + nn] = __uint_as_float(r[j]);
+      for (int j = 0; j < 16; ++j, to += n) *to = __uint_as_float(r[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j, to += n)
+        if (c + j < tile.count) *to = __uint_as_float(r[j]);
+    }
   }
 }
 
@@ -214,8 +221,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 // ---- tiles of 256 rows: persistent CTA pairs (gemm_pair.cuh) ------------------------
 // A prompt's products are bound by the tensor cores like its projections, and the tiles of the list are of unequal size: the pairs go from tile to tile,
 // entries without rows cost nothing and a tile with fewer rows takes as many columns as it has (in steps of 32). Measured against one CTA per two weight
-// tiles and 256 rows, up and down: 7006 rows, width 2048, 16 experts of 1408 and a shared one of 2816: 343 + 160 -> 210 + 131 us; 2048 rows, experts
-// of 2112 without gates, a shared one of 4224: 115 + 80 -> 78 + 71.
+// tiles and 256 rows, up and down, launches back to back: 7006 rows, width 2048, 16 experts of 1408 and a shared one of 2816: 289 + 151 -> 235 + 136 us;
+// 2048 rows, experts of 2112 without gates, a shared one of 4224: 123 + 85 -> 88 + 70; 7006 rows, width 1024, 64 experts of 512: 150 + 94 -> 115 + 72.
 template <int GATED>
 struct MixtureWork {
   static constexpr uint32_t kBatch = GATED ? 2 : 4;

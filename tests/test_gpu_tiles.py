@@ -57,3 +57,19 @@ def test_mixtures_of_decode_batches(pkg, backend, design, shape, rows):
     longer k."""
     oracle_of, cfg, w = mixture(design, *shape, seed=rows)
     check(pkg, backend, oracle_of, cfg, w, np.random.default_rng(rows).integers(0, 64, rows).tolist())
+
+
+def uneven(rng, rows):
+    """Tokens so unequal in number that experts get one row, a few, about one tile, several tiles or none."""
+    t = np.repeat([0, 1, 2, 3, 4], [257, 33, 31, 1, rows - 322])
+    rng.shuffle(t)
+    return t.tolist()
+
+
+@pytest.mark.parametrize("shape", [(200, 5, 1, 3080, 600), (2568, 5, 1, 72, 136), (72, 4, 1, 3080, 3080)])
+@pytest.mark.parametrize("design", ["zulozen", "belizen", "vusenex"])
+def test_mixtures_of_several_rounds(pkg, backend, design, shape):
+    """Tiles of 256 rows, more than two rounds of the 74 pairs: both accumulators, rings that go on from a tile of one width to one of another, entries
+    without rows between others, a pair that comes from the shared expert to the others."""
+    oracle_of, cfg, w = mixture(design, *shape, seed=7)
+    check(pkg, backend, oracle_of, cfg, w, uneven(np.random.default_rng(8), 1100))
