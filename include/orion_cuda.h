@@ -249,6 +249,11 @@ int orion_cuda_selftest_peer_wait(OrionBackend *backend, uint64_t limit_us, uint
  * to know whether one of its launches timed out synchronises its stream and calls this. */
 int orion_cuda_poll_wait_timeouts(OrionBackend *backend, uint32_t *mask);
 
+/* Failure-detection self-test (no reference counterpart): sets the time-out words of `mask` (bits as above) as a bounded wait
+ * that gives up sets them, without one. The next step of a bf16 model that uses such a kernel family must fail with
+ * EngineError::Backend, and the step after it must not. */
+int orion_cuda_selftest_set_wait_timeouts(OrionBackend *backend, uint32_t mask);
+
 /* CheckpointLoader::open + ModelWeights::load for a whole directory
  * (crates/orion-models/src/loader.rs:112-235, transformer.rs:62-120,180-205): every
  * `*.safetensors` file in name order (the first file wins for a duplicated tensor name),

@@ -61,6 +61,17 @@ class CudaBackend:
         check(_ffi.lib().orion_cuda_selftest_bounded_wait(self._h, limit_us, C.byref(t), C.byref(w)))
         return bool(t.value), int(w.value)
 
+    def selftest_set_wait_timeouts(self, mask: int) -> None:
+        """Sets the time-out words of ``mask`` as a device wait that gave up would; bits as in ``poll_wait_timeouts``."""
+        check(_ffi.lib().orion_cuda_selftest_set_wait_timeouts(self._h, mask))
+
+    def poll_wait_timeouts(self) -> int:
+        """Reads and clears the device's time-out words: bit 0 projections, 1 decode attention, 2 prefill attention, 3 tensor-parallel hand-over,
+        4 mixtures of experts, 5 gated linear attention."""
+        mask = C.c_uint32()
+        check(_ffi.lib().orion_cuda_poll_wait_timeouts(self._h, C.byref(mask)))
+        return int(mask.value)
+
     def selftest_peer_wait(self, limit_us: int):
         """The same for the peer polls of the tensor-parallel hand-over (inbox units that no peer
         ever writes); returns ``(timed_out, waited_us)``."""

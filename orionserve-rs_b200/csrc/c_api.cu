@@ -561,6 +561,18 @@ int orion_cuda_poll_wait_timeouts(OrionBackend *backend, uint32_t *mask) {
   return ORION_OK;
 }
 
+int orion_cuda_selftest_set_wait_timeouts(OrionBackend *backend, uint32_t mask) {
+  orion::clear_error();
+  ORION_TRY(orion::check_backend(backend));
+  const void *words[6] = {orion::gemm_tc_error_word(), orion::decode_error_word(), orion::prefill_error_word(),
+                          orion::tp_error_word(),      orion::moe_error_word(),    orion::gla_error_word()};
+  if (mask >> 6) return orion::set_error(ORION_ERR_INVALID_REQUEST, "time-out mask %#x has unknown bits", mask);
+  const uint32_t one = 1;
+  for (int i = 0; i < 6; ++i)
+    if (mask >> i & 1u) ORION_CUDA_CHECK("time-out word", cudaMemcpy(const_cast<void *>(words[i]), &one, sizeof one, cudaMemcpyHostToDevice));
+  return ORION_OK;
+}
+
 int orion_cuda_model_load_checkpoint(OrionModel *model, const char *directory, uint64_t *tensors_loaded) {
   clear_error();
   if (!model) return set_error(ORION_ERR_INVALID_REQUEST, "null model handle");

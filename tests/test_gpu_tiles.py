@@ -73,3 +73,57 @@ def test_mixtures_of_several_rounds(pkg, backend, design, shape):
     without rows between others, a pair that comes from the shared expert to the others."""
     oracle_of, cfg, w = mixture(design, *shape, seed=7)
     check(pkg, backend, oracle_of, cfg, w, uneven(np.random.default_rng(8), 1100))
+
+
+@pytest.mark.parametrize("rows", [257, 300, 513])
+@pytest.mark.parametrize("design", ["metapel", "zulozen", "belizen"])
+def test_feed_forwards_of_many_rows(pkg, backend, design, rows):
+    """GELU, the square of ReLU with a bias, and GeGLU in the epilogue of the pairs: 6416 columns are more than one round, with the last tiles in pieces."""
+    if design == "metapel":
+        oracle_of, cfg = metapel, metapel_models.config(128, 64, [metapel_models.mingru(64, 6416)])
+        w = silence(metapel_models.random_weights(cfg, seed=rows), "mix.o")
+    elif design == "zulozen":
+        oracle_of, cfg = zulozen, zulozen_models.config(128, 64, [zulozen_models.attn(1, 1, 8, 8, 4, zulozen_models.dense(6416))])
+        w = silence(zulozen_models.random_weights(cfg, seed=rows), "mix.o")
+    else:
+        oracle_of, cfg = belizen, belizen_models.config(128, 64, [belizen_models.gla(1, 8, 8, 4.0, 2, belizen_models.dense(3208))])
+        w = silence(belizen_models.random_weights(cfg, seed=rows), "mix.o")
+    check(pkg, backend, oracle_of, cfg, w, np.random.default_rng(rows).integers(0, 64, rows).tolist())
+
+
+@pytest.mark.parametrize("rows", [257, 513])
+def test_swiglu_of_many_rows(pkg, backend, oracle, rows):
+    """The same for SwiGLU, in a Llama layer."""
+    desc = dict(hidden_size=128, num_layers=1, num_attention_heads=2, num_kv_heads=1, head_dim=64, vocab_size=64, ffn_dim=3208, max_position_embeddings=640,
+                rope_theta=10000.0, rms_norm_eps=1e-5, has_qkv_bias=False, tied_lm_head=False, num_blocks=40, block_size=16)
+    t = {k: (oracle.round_to_bf16(v) if v.ndim == 2 else v) for k, v in random_tensors(np.random.default_rng(rows), desc, std=0.1).items()}
+    ref = oracle.Model(**desc).load(t)
+    meta = pkg.ModelMetadata(architecture="llama", name="s", **{k: v for k, v in desc.items() if k not in ("num_blocks", "block_size")})
+    dev = pkg.CudaTransformerModel.new(meta, t, 40, 16, backend, compute_dtype=pkg.DType.BF16, max_batch_tokens=640, max_batch_sequences=2)
+    toks, table = np.random.default_rng(1).integers(0, 64, rows).tolist(), [list(range(40))]
+    oracle.set_threads(8)
+    exp = ref.forward(oracle.Batch(toks, list(range(rows)), [rows], [rows], table))
+    oracle.set_threads(1)
+    got = dev.forward(pkg.ForwardBatch(toks, list(range(rows)), [1], [rows], [rows], table, has_prefill=True)).logits
+    assert worst_error(got, exp) < TOL
+
+
+@pytest.mark.parametrize("scale", [-0.25, 0.25])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 2, 64, 64), (8, 1, 128, 128), (4, 2, 64, 128)])
+@pytest.mark.parametrize("design", ["zulozen", "belizen, capped", "belizen"])
+def test_scales_of_either_sign(pkg, backend, design, heads, kv_heads, dim, vdim, scale):
+    """Scores that a negative scale turns round: prompts, portions and single tokens, with masks and sinks, with soft caps and without."""
+    if design == "zulozen":
+        oracle_of, m = zulozen, zulozen_models
+        cfg = m.config(96, 40, [m.attn(heads, kv_heads, dim, vdim, 90, scale=scale)])
+    else:
+        oracle_of, m = belizen, belizen_models
+        cfg = m.config(96, 40, [m.attn(heads, kv_heads, dim, vdim, 90, 3, scale=scale, cap=20.0 if "capped" in design else 0.0)])
+    w = m.random_weights(cfg, seed=5)
+    t = np.random.default_rng(2).integers(0, 40, 230).tolist()
+    exp = oracle_of.forward(t, cfg, w)
+    turned = dict(cfg, layers=[dict(e, mixer=dict(e["mixer"], scale=-scale)) for e in cfg["layers"]])
+    assert worst_error(oracle_of.forward(t, turned, w), exp) > 3 * TOL  # the sign shows
+    f = Feeder(pkg, make_model(pkg, backend, cfg, w, pkg.DType.BF16))
+    assert worst_error(f.run("p", t, [230]), exp) < TOL
+    assert worst_error(f.run("q", t, [130, 37, 1]), exp) < TOL
