@@ -60,9 +60,9 @@ __device__ __forceinline__ void gtrace(uint32_t slot, int k) {
 // the weight bytes in flight per SM (160 KiB -> 6.0 TB/s, 128 KiB -> 5.3 TB/s), so shared
 // memory goes to the W ring first.
 // MT = weight tiles of 128 rows per CTA. Decode batches stream weights (MT = 1, as many CTAs as
-// possible); prefill batches are tensor-bound and limited by the shared-memory fill rate, so a
-// CTA there takes two weight tiles against one activation tile (MT = 2: 64 KiB of operands per
-// 2.1 MFLOP instead of 48 KiB per 1.05), with two accumulators in tensor memory.
+// possible); 129 to 256 rows feel the shared-memory fill rate as well, so a CTA there takes two weight
+// tiles against one activation tile (MT = 2: 64 KiB of operands per 8.4 MFLOP instead of 48 KiB per 4.2),
+// with two accumulators in tensor memory.
 template <int TOKN, int WST, int XST, int MT = 1>
 struct TcConfig {
   static constexpr int kWBytes = MT * kTileN * kSlabK * 2;
@@ -101,8 +101,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_ready + 1);
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const TileXy tile = gridDim.y == 1 ? TileXy{blockIdx.x, 0} : raster(blockIdx.y * gridDim.x + blockIdx.x, gridDim.x, gridDim.y);
-  const uint32_t n0 = tile.x * (MT * kTileN), t0 = tile.y * TOKN, split = blockIdx.z;
+  const uint32_t n0 = blockIdx.x * (MT * kTileN), t0 = blockIdx.y * TOKN, split = blockIdx.z;
   const uint32_t nkb = (K + kSlabK - 1) / kSlabK;
   const uint32_t kb_begin = (uint32_t)((uint64_t)split * nkb / splits);
   const uint32_t kb_end = (uint32_t)((uint64_t)(split + 1) * nkb / splits);
@@ -556,38 +555,20 @@ int launch_pair(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float 
   return form(x, ldx, w, ldw, partial, act, rows, n, k, splits, ldc, epi, stream, ready, bias);
 }
 
-// Who takes the persistent pairs: 1 (default) = batches of more than 256 rows, 2 = of more than 128 (the parity tests run this), 0 = nobody.
-// ORION_GEMM_PAIR overrides. The four projections of the 8B shape at 512 / 2048 / 8192 rows, f32 out: 188 / 611 / 2380 us with pairs, 239 / 775 / 2540
-// with one CTA per 256-token tile. At 129 to 256 rows the two are equal: the wider gate/up 3-6 % slower with pairs, the others 5-13 % faster.
+// Who takes the persistent pairs: batches of more than 256 rows, with ORION_GEMM_PAIR=2 of more than 128 (the parity tests run this). The four
+// projections of the 8B shape at 512 / 2048 / 8192 rows, f32 out: 188 / 611 / 2380 us with pairs, 239 / 775 / 2540 with one CTA per 256-token tile. At 129 to
+// 256 rows the two are equal: the wider gate/up 3-6 % slower with pairs, the others 5-13 % faster.
 // Matrices of one weight tile (routers) are the exception: the second CTA of a pair has nothing but padding, and with more than kRouterRows tokens single
 // CTAs are faster. 16 rows of k 2048 and the norm that reads the result, 2048 / 3000 / 4096 / 8192 tokens: single CTAs 12.0 / 12.6 / 13.6 / 19.5 us, pairs
 // with the best k splits 11.1 / 12.8 / 15.3 / 23.1; 64 rows of k 4096: 14.7 / 15.4 / 16.3 / 21.4 and 12.2 / 14.6 / 17.3 / 25.3.
-int g_gemm_pair = std::getenv("ORION_GEMM_PAIR") ? std::atoi(std::getenv("ORION_GEMM_PAIR")) : 1;
+const uint32_t g_pair_rows = std::getenv("ORION_GEMM_PAIR") && std::atoi(std::getenv("ORION_GEMM_PAIR")) >= 2 ? 128 : 256;
 constexpr uint32_t kRouterRows = 3072;
-bool takes_pairs(uint32_t rows, uint32_t n) {
-  return g_gemm_pair >= 1 && rows > (g_gemm_pair >= 2 ? 128u : 256u) && (n > (uint32_t)kTileN || rows <= kRouterRows);
-}
+bool takes_pairs(uint32_t rows, uint32_t n) { return rows > g_pair_rows && (n > (uint32_t)kTileN || rows <= kRouterRows); }
 
-// Tuning A/B: ORION_GEMM_PREFILL_TILES=1 keeps one weight tile per CTA for prefill-sized batches
-// (two tiles measured 3 % faster on the continuous-batching workload, gate/up only: the other
-// projections have too few tiles to halve their grid).
-int g_prefill_tiles = std::getenv("ORION_GEMM_PREFILL_TILES") ? std::atoi(std::getenv("ORION_GEMM_PREFILL_TILES")) : 2;
-// How a prefill-sized projection with fewer than 148 tiles of 256 tokens reaches every SM: 2 = k
-// splits (default), 1 = 128-token tiles, 0 = not at all. Measured on the continuous-batching
-// workload at the 8B shape: 12.07 / 12.46 / 12.32 s. ORION_GEMM_PREFILL_FILL overrides.
-int g_prefill_fill = std::getenv("ORION_GEMM_PREFILL_FILL") ? std::atoi(std::getenv("ORION_GEMM_PREFILL_FILL")) : 2;
-// Weight tiles per CTA for a prefill-sized batch: two share one activation tile (less shared-memory
-// fill per flop). Mode 2 (default): only where the grid stays full without k splits; mode 3: always
-// (measured no better on the continuous-batching workload: 12.19 vs 11.94 s).
 // Batches of 129..256 rows stream weights like decode but already feel the fill rate (48 KiB of operands per
-// 4.2 MFLOP with one weight tile): ORION_GEMM_MID_MT=2 (default) gives a CTA two weight tiles there too.
+// 4.2 MFLOP with one weight tile): ORION_GEMM_MID_MT=2 (default) gives a CTA two weight tiles there, 1 one.
 int g_mid_mt = std::getenv("ORION_GEMM_MID_MT") ? std::atoi(std::getenv("ORION_GEMM_MID_MT")) : 2;
-uint32_t prefill_weight_tiles(uint32_t rows, uint32_t n) {
-  if (rows > 128 && rows <= 256) return g_mid_mt >= 2 && n >= 2 * (uint32_t)kTileN ? 2 : 1;
-  if (rows <= 256 || g_prefill_tiles < 2) return 1;
-  if (g_prefill_tiles >= 3) return 2;
-  return ((n + kTileN - 1) / kTileN) * ((rows + 255) / 256) >= 296 ? 2 : 1;
-}
+uint32_t weight_tiles_per_cta(uint32_t rows, uint32_t n) { return rows > 128 && rows <= 256 && g_mid_mt >= 2 && n >= 2 * (uint32_t)kTileN ? 2 : 1; }
 int g_small_stages = 5;  // 5: deep weight ring + short activation ring for decode batches; 4: equal rings
 // Batches of 65..128 rows: 0 (default) = 4 weight + 2 activation stages, 96 KiB, two CTAs per SM like the
 // smaller tiles (the split-K planner counts on two); 1 = 6 + 6 stages, 192 KiB, one CTA per SM, k splits
@@ -625,9 +606,7 @@ int launch_gemm_tc(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, flo
   if (splits < 1 || splits > nkb)
     return set_error(ORION_ERR_INTERNAL, "gemm split count %u outside 1..%u", splits, nkb);
   const bool deep = g_small_stages >= 5;
-  uint32_t tt = token_tile(rows);
-  // prefill batches whose 256-token tiles would leave SMs idle take 128-token tiles instead
-  if (rows > 256 && g_prefill_fill == 1 && ((n + kTileN - 1) / kTileN) * ((rows + 255) / 256) < 148) tt = 128;
+  const uint32_t tt = token_tile(rows);
   if (takes_pairs(rows, n) && !cluster_reduce) {
     if (splits > (k + PairConfig::kStageK - 1) / PairConfig::kStageK) return set_error(ORION_ERR_INTERNAL, "gemm split count %u leaves a split empty", splits);
     return launch_pair(x, ldx, w, ldw, partial, act, rows, n, k, splits, ldc, epi, stream, ready, bias);
@@ -647,7 +626,7 @@ int launch_gemm_tc(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, flo
                  ? launch_tc<128, 4, 2>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias)
                  : launch_tc<128, 6, 6>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias);
     default: {
-      const uint32_t mt = (!cluster_reduce && prefill_weight_tiles(rows, n) == 2) ? 2 : 1;
+      const uint32_t mt = cluster_reduce ? 1 : weight_tiles_per_cta(rows, n);
       return mt == 2 ? launch_tc<256, 3, 3, 2>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias)
                      : launch_tc<256, 4, 4>(x, ldx, w, ldw, partial, act, rows, n, k, splits, cluster_reduce, ldc, epi, stream, ready, bias);
     }
@@ -718,25 +697,14 @@ GemmPlan gemm_plan(bool is_bf16, uint32_t rows, uint32_t n, uint32_t k, uint32_t
     p.splits = p.out_slabs = pair_splits(rows, n, k);
     return p;
   }
-  if (rows > 256) {
-    // Prefill-sized batches are tensor-bound; the 256-token tiles take a whole SM each (192 KiB of
-    // rings), so a projection with few weight tiles (N = 4096: 32) needs k splits to reach all SMs.
-    const uint32_t rows_per_cta = kTileN * prefill_weight_tiles(rows, n);
-    const uint32_t big = ((n + rows_per_cta - 1) / rows_per_cta) * ((rows + 255) / 256);
-    const uint32_t nkb_big = (k + kSlabK - 1) / kSlabK;
-    if (big < 148 && g_prefill_fill == 2) {
-      uint32_t s = 296 / big;
-      const uint32_t cap = nkb_big / 8 ? nkb_big / 8 : 1;  // at least eight k slabs per split
-      if (s > cap) s = cap;
-      if (s > 4) s = 4;
-      p.splits = p.out_slabs = s < 1 ? 1 : s;
-    }
-    (void)nkb_big;
+  const uint32_t nkb = (k + kSlabK - 1) / kSlabK;
+  if (rows > 256) {  // one weight tile and many tokens: up to four k splits of at least eight slabs, in at most two waves
+    const uint32_t tiles = (rows + 255) / 256;
+    if (tiles < 148) p.splits = p.out_slabs = std::max(1u, std::min({296 / tiles, nkb / 8, 4u}));
     return p;
   }
-  const uint32_t rows_per_cta = kTileN * (g_cluster_splitk ? 1 : prefill_weight_tiles(rows, n));
+  const uint32_t rows_per_cta = kTileN * (g_cluster_splitk ? 1 : weight_tiles_per_cta(rows, n));
   const uint32_t tiles = ((n + rows_per_cta - 1) / rows_per_cta) * ((rows + token_tile(rows) - 1) / token_tile(rows));
-  const uint32_t nkb = (k + kSlabK - 1) / kSlabK;
   // the 256-token tile (and the 6 + 6 stage 128-token one) fills an SM by itself: one wave is 148 CTAs
   const bool one_per_sm = g_mid_tile != 2 && (token_tile(rows) == 256 || (token_tile(rows) == 128 && g_mid_tile == 1));
   uint32_t s = (one_per_sm ? g_target_ctas / 2 : g_target_ctas) / (tiles ? tiles : 1);

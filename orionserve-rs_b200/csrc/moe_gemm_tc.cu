@@ -1,14 +1,15 @@
-// Grouped products of a mixture of experts on the 5th-generation tensor cores (bf16): the projection kernel of gemm_tc.cu over
+// Grouped products of a mixture of experts on the 5th-generation tensor cores (bf16): the projection kernels of gemm_tc.cu over
 // a list of tiles, each a run of rows that share one expert. As there, the weight matrix is the M operand (128 rows per
-// MMA) and the rows are N, so an expert's weights are streamed once per tile, whatever the number of its rows; a tile's rows
-// past its count belong to the next expert and are not stored.
-//   CTA (x: weight tiles; y: row tile, the shared expert's first; z: k split), 256 threads
+// MMA, 256 in a pair of CTAs) and the rows are N, so an expert's weights are streamed once per tile, whatever the number of its rows; a tile's
+// rows past its count belong to the next expert and are not stored. The epilogue stores f32 rows, or f(w g) * (w u), f a gated activation, of
+// neighbouring gate and up rows with the row's score w, or an activation f(w u) without a gate.
+// Tiles of up to 128 rows (moe_gemm_tc_kernel): a CTA (x: weight tile; y: row tile, the shared expert's first; z: k split) of 256 threads
 //   warp 0     one lane streams the expert's weights by TMA, 64-wide k slabs, 128-byte swizzled (the shared expert's before the
 //              preceding kernel has ended; the others once the tile list is there)
 //   warp 2     one lane does the same with the tile's rows
 //   warp 1     allocates tensor memory, one lane issues the MMAs
-//   warps 4-7  epilogue (all eight warps where an activation is computed): f32 rows, or f(w g) * (w u), f a gated activation, of neighbouring gate and up rows with the row's score w, or
-//              an activation f(w u) without a gate
+//   warps 4-7  epilogue (all eight warps where an activation is computed)
+// Tiles of 256 rows (moe_pair_kernel): persistent CTA pairs, see gemm_pair.cuh.
 // Every wait is bounded; a wait that runs out sets the device error word and the CTA still frees its tensor memory.
 #include "gemm_pair.cuh"
 #include "value_cache.h"
@@ -23,13 +24,13 @@ constexpr uint32_t kTileN = 128, kSlabK = 64, kThreads = 256, kSms = 148;
 
 __device__ uint32_t g_moe_error = 0;
 
-// WST / XST: stages of the weight and the row ring; MT: weight tiles per CTA.
-template <int TOKN, int WST, int XST, int MT>
+// WST / XST: stages of the weight and the row ring.
+template <int TOKN, int WST, int XST>
 struct MoeConfig {
-  static constexpr int kWBytes = MT * kTileN * kSlabK * 2, kXBytes = TOKN * kSlabK * 2;
+  static constexpr int kWBytes = kTileN * kSlabK * 2, kXBytes = TOKN * kSlabK * 2;
   static constexpr int kXOffset = WST * kWBytes, kBarOffset = kXOffset + XST * kXBytes;
   static constexpr int kSmemBytes = kBarOffset + 1024 + 256;
-  static constexpr uint32_t kTmemCols = MT * TOKN < 32 ? 32 : MT * TOKN;
+  static constexpr uint32_t kTmemCols = TOKN < 32 ? 32 : TOKN;
   static_assert(kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0 && kSmemBytes <= 232448, "tile does not fit an SM");
 };
 
@@ -93,11 +94,11 @@ __device__ __forceinline__ void store_chunk(const TcArgs &a, bool shared, const 
 }
 
 // GATED: 0 = f32 products, 1 = SwiGLU, 2 = the gated activations of the arguments, 3 = no gate, the exact GELU of every product.
-template <int TOKN, int WST, int XST, int MT, int GATED>
+template <int TOKN, int WST, int XST, int GATED>
 __global__ void __launch_bounds__(kThreads)
 moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_sw,
                    const __grid_constant__ CUtensorMap map_sx, TcArgs a) {
-  using Cfg = MoeConfig<TOKN, WST, XST, MT>;
+  using Cfg = MoeConfig<TOKN, WST, XST>;
   extern __shared__ uint8_t raw_smem[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
   uint8_t *w_ring = smem, *x_ring = smem + Cfg::kXOffset;
@@ -106,7 +107,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_ready + 1);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool shared = blockIdx.y < a.shared_tiles;
-  const uint32_t n = shared ? a.shared_n : a.n, k = shared ? a.shared_k : a.k, n0 = blockIdx.x * (MT * kTileN), split = blockIdx.z;
+  const uint32_t n = shared ? a.shared_n : a.n, k = shared ? a.shared_k : a.k, n0 = blockIdx.x * kTileN, split = blockIdx.z;
   if (n0 >= n) return;  // the grid is as wide as the wider of the two products
   if (threadIdx.x == 0) {
     for (int s = 0; s < WST; ++s) mbar_init(&full_w[s], 1), mbar_init(&empty_w[s], 1);
@@ -144,10 +145,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint32_t s = i % WST;
         if (!mbar_wait(&empty_w[s], ((i / WST) & 1) ^ 1)) { ok = false; break; }
         mbar_arrive_expect_tx(&full_w[s], Cfg::kWBytes);
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)  // rows past the matrix read as zeros, rows past the expert belong to the next one
-          tma_load_2d(w_ring + s * Cfg::kWBytes + mt * (kTileN * kSlabK * 2), mw, (int)((kb_begin + i) * kSlabK),
-                      (int)(tile.expert * n + n0 + mt * kTileN), &full_w[s]);
+        // rows past the matrix read as zeros, rows past the expert belong to the next one
+        tma_load_2d(w_ring + s * Cfg::kWBytes, mw, (int)((kb_begin + i) * kSlabK), (int)(tile.expert * n + n0), &full_w[s]);
       }
     }
   } else if (warp == 2) {
@@ -170,9 +169,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint32_t wt = smem_u32(w_ring + sw * Cfg::kWBytes), xt = smem_u32(x_ring + sx * Cfg::kXBytes);
 #pragma unroll
         for (uint32_t kk = 0; kk < kSlabK / 16; ++kk)
-#pragma unroll
-          for (int mt = 0; mt < MT; ++mt)
-            umma_bf16(tmem_base + mt * TOKN, desc_k_sw128(wt + mt * (kTileN * kSlabK * 2) + kk * 32), desc_k_sw128(xt + kk * 32), id, (i > 0 || kk > 0) ? 1u : 0u);
+          umma_bf16(tmem_base, desc_k_sw128(wt + kk * 32), desc_k_sw128(xt + kk * 32), id, (i > 0 || kk > 0) ? 1u : 0u);
         umma_commit(&empty_w[sw]);
         umma_commit(&empty_x[sx]);
       }
@@ -191,7 +188,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tc_fence_after();
     constexpr int kBatch = TOKN >= 64 ? (GATED ? 2 : 4) : (GATED ? 1 : TOKN / 16);
 #pragma unroll 1
-    for (int mb = kGroups == 2 && warp < 4 ? 16 * kBatch : 0; mb < MT * TOKN; mb += 16 * kBatch * kGroups) {
+    for (int mb = kGroups == 2 && warp < 4 ? 16 * kBatch : 0; mb < TOKN; mb += 16 * kBatch * kGroups) {
       uint32_t rr[kBatch][16];
       if (ok && my_kb > 0) {
 #pragma unroll
@@ -205,8 +202,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       }
 #pragma unroll
       for (int b = 0; b < kBatch; ++b) {
-        const int mc = mb + 16 * b;
-        const uint32_t c = mc % TOKN, nn = n0 + (mc / TOKN) * kTileN + lq * 32 + lane;  // first row of the tile in this chunk, weight row
+        const uint32_t c = mb + 16 * b, nn = n0 + lq * 32 + lane;  // first row of the tile in this chunk, weight row
         if (c >= tile.count) continue;  // warp-uniform
         store_chunk<GATED>(a, shared, tile, n, nn, c, rr[b], split);
       }
@@ -289,9 +285,9 @@ int product_form(const MoeProduct &p, bool gated) {
   return !gated ? 0 : (p.f.plain() ? 3 : (p.f.kind == kGatedSilu && p.shared_f.kind == kGatedSilu ? 1 : 2));
 }
 
-template <int TOKN, int WST, int XST, int MT>
+template <int TOKN, int WST, int XST>
 int launch_product(const MoeProduct &p, bool swiglu, uint32_t splits, MoePlan plan, cudaStream_t stream) {
-  using Cfg = MoeConfig<TOKN, WST, XST, MT>;
+  using Cfg = MoeConfig<TOKN, WST, XST>;
   CUtensorMap mw, mx, msw, msx;
   ORION_TRY(matrix_map(p.w, (uint64_t)p.experts * p.n, p.k, kTileN, &mw));
   ORION_TRY(matrix_map(p.x, p.sorted_rows, p.k, TOKN, &mx));
@@ -302,13 +298,13 @@ int launch_product(const MoeProduct &p, bool swiglu, uint32_t splits, MoePlan pl
   }
   const uint32_t shared_tiles = p.shared_n ? (p.rows + TOKN - 1) / TOKN : 0;
   const TcArgs a{p.n, p.k, p.shared_n, p.shared_k, shared_tiles, p.rows, p.sorted_rows, splits, p.tiles, p.row_score, p.act, p.shared_act, p.out, p.shared_out, p.f, p.shared_f};
-  const dim3 grid((std::max(p.n, p.shared_n) + MT * kTileN - 1) / (MT * kTileN), shared_tiles + plan.tiles, splits);
+  const dim3 grid((std::max(p.n, p.shared_n) + kTileN - 1) / kTileN, shared_tiles + plan.tiles, splits);
   static bool attr_set[4][kMaxDeviceOrdinals] = {};
   const int form = product_form(p, swiglu);
-  auto kernel = form == 0   ? moe_gemm_tc_kernel<TOKN, WST, XST, MT, 0>
-                : form == 1 ? moe_gemm_tc_kernel<TOKN, WST, XST, MT, 1>
-                : form == 2 ? moe_gemm_tc_kernel<TOKN, WST, XST, MT, 2>
-                            : moe_gemm_tc_kernel<TOKN, WST, XST, MT, 3>;
+  auto kernel = form == 0   ? moe_gemm_tc_kernel<TOKN, WST, XST, 0>
+                : form == 1 ? moe_gemm_tc_kernel<TOKN, WST, XST, 1>
+                : form == 2 ? moe_gemm_tc_kernel<TOKN, WST, XST, 2>
+                            : moe_gemm_tc_kernel<TOKN, WST, XST, 3>;
   ORION_CUDA_CHECK("moe_gemm attr", ensure_dynamic_smem(kernel, Cfg::kSmemBytes, attr_set[form]));
   ORION_CUDA_CHECK("moe_gemm", launch_pdl(kernel, grid, dim3(kThreads), (size_t)Cfg::kSmemBytes, stream, mw, mx, msw, msx, a));
   count_launch();
@@ -364,10 +360,10 @@ int launch_moe_product_tc(const MoeProduct &p, bool swiglu, uint32_t splits, Moe
   if (swiglu && splits != 1) return set_error(ORION_ERR_INTERNAL, "the fused SwiGLU epilogue needs one k split");
   const bool three = plan.tile_rows <= 32 && three_to_an_sm(p, splits, plan);
   switch (plan.tile_rows) {
-    case 16: return three ? launch_product<16, 4, 3, 1>(p, swiglu, splits, plan, stream) : launch_product<16, 6, 3, 1>(p, swiglu, splits, plan, stream);
-    case 32: return three ? launch_product<32, 4, 2, 1>(p, swiglu, splits, plan, stream) : launch_product<32, 6, 3, 1>(p, swiglu, splits, plan, stream);
-    case 64: return launch_product<64, 5, 3, 1>(p, swiglu, splits, plan, stream);
-    case 128: return launch_product<128, 4, 2, 1>(p, swiglu, splits, plan, stream);
+    case 16: return three ? launch_product<16, 4, 3>(p, swiglu, splits, plan, stream) : launch_product<16, 6, 3>(p, swiglu, splits, plan, stream);
+    case 32: return three ? launch_product<32, 4, 2>(p, swiglu, splits, plan, stream) : launch_product<32, 6, 3>(p, swiglu, splits, plan, stream);
+    case 64: return launch_product<64, 5, 3>(p, swiglu, splits, plan, stream);
+    case 128: return launch_product<128, 4, 2>(p, swiglu, splits, plan, stream);
     default: return launch_pairs(p, swiglu, splits, plan, stream);
   }
 }

@@ -92,10 +92,9 @@ def test_linear_f32_is_bit_exact(pkg, backend, oracle, kats):
                                       (129, 640, 1024), (300, 1152, 2048), (8, 200, 72),
                                       # prefill-sized batches: two weight tiles per CTA, ragged last tile
                                       (512, 384, 512), (260, 128, 64), (700, 2176, 256),
-                                      # an even number of weight tile groups: CTA pairs (cta_group::2), one and two weight
-                                      # tiles per CTA, ragged last token tile (one CTA's half entirely past the end), ragged
-                                      # last weight tile
-                                      # (from 4096 rows on by default, everywhere the grid allows in the paired re-run below)
+                                      # CTA pairs (cta_group::2): ragged last token tile (one CTA's half entirely past the
+                                      # end), ragged last weight tile (more than 256 rows by default, more than 128 in the
+                                      # paired re-run below)
                                       (300, 1024, 2048), (200, 1024, 512), (600, 1000, 1024), (300, 19456, 256),
                                       (4100, 512, 256),
                                       # Llama-3-70B projections on one of 8 ranks: qkv, o, gate|up, down
@@ -668,9 +667,9 @@ def test_qwen2_7b_head_layout_with_qkv_bias_on_the_tuned_bf16_path(pkg, backend,
 
 
 def test_paired_gemm_variant_matches_the_oracle(pkg, backend):
-    """256-token GEMM tiles as CTA pairs (tcgen05 cta_group::2) are used from 4096 rows on by default; the
-    switch is read when the library loads, so the parity cases with 129 rows and more run once more in a
-    child process with pairs wherever the grid allows: plain and SwiGLU epilogues, one and two weight tiles."""
+    """Persistent CTA pairs (tcgen05 cta_group::2) take projections of more than 256 rows by default; the switch is read
+    when the library loads, so the parity cases run once more in a child process with pairs from 129 rows on: plain and
+    SwiGLU epilogues."""
     import os
     import subprocess
     import sys
