@@ -220,10 +220,10 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
     }
   } else if (warp >= 4) {
     // Epilogue: warp w reads tensor-memory lanes 32 * (w % 4) .. + 31 (lane = weight row, column = token); the two warps of the same lanes take
-    // turns, a batch of columns each.
+    // turns, 16 columns each. With two or four loads of 16 in flight the loop was that much longer, and the eight warps waited for instructions: GELU of
+    // 512 x 8192, k 512, four at a time 22.5 us, two 20.2, one 18.4; with all activations in one kernel, told apart for every value, 23.0.
     // The output may still be read by the kernel before the producer of x. (With a ready counter the producer has read it before it counted.)
     if (!ready.counter) pdl_wait();
-    constexpr uint32_t kBatch = Work::kBatch;  // 16-column loads in flight before one wait
     uint32_t turn = 0;
     for (uint32_t t = pair; ok && t < total; t += pairs) {
       const typename Work::Job j = work.job(t);
@@ -232,8 +232,8 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
       if (!wait(&acc_full[buf], (turn >> 1) & 1)) { ok = false; break; }
       ++turn;
       tc_fence_after();
-      constexpr uint32_t kStep = 16 * kBatch * (Cfg::kEpilogueWarps / 4);
-      uint32_t mb = 16 * kBatch * ((warp - 4) / 4);
+      constexpr uint32_t kStep = 16 * (Cfg::kEpilogueWarps / 4);
+      uint32_t mb = 16 * ((warp - 4) / 4);
       // once this warp's last columns are in registers, the MMAs of the tile after the next may write them
       auto release = [&] {
         tc_fence_before();
@@ -243,15 +243,11 @@ __device__ __forceinline__ void run_pairs(const Work &work, ReadyWait ready, uin
       if (mb >= j.cols) release();
 #pragma unroll 1
       for (; mb < j.cols; mb += kStep) {
-        uint32_t rr[kBatch][16];
-#pragma unroll
-        for (uint32_t b = 0; b < kBatch; ++b)
-          if (mb + 16 * b < j.cols) tmem_ld16(acc + mb + 16 * b, rr[b]);
+        uint32_t rr[16];
+        tmem_ld16(acc + mb, rr);
         tmem_ld_wait();
         if (mb + kStep >= j.cols) release();
-#pragma unroll
-        for (uint32_t b = 0; b < kBatch; ++b)
-          if (mb + 16 * b < j.cols) work.store(j, rank * Cfg::kRows + (warp & 3) * 32 + lane, mb + 16 * b, rr[b]);
+        work.store(j, rank * Cfg::kRows + (warp & 3) * 32 + lane, mb, rr);
       }
     }
   }

@@ -349,11 +349,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
 // ---- many rows: persistent CTA pairs (gemm_pair.cuh) ------------------------------
 
-enum PairOutput : int { kPairPartials = 0, kPairSwiglu = 1, kPairAct = 2 };
-
-template <int OUT>
+template <GemmEpilogue OUT>
 struct ProjectionWork {
-  static constexpr uint32_t kBatch = 4;
   static constexpr bool kStaticTiles = true;
   struct Job : PairJob {
     float *out;
@@ -362,7 +359,7 @@ struct ProjectionWork {
   float *partial;
   bf16 *act;
   const float *bias;
-  uint32_t M, N, splits, tokn, whole, tail, ldc, epilogue, tiles_x, tiles_y, stages;
+  uint32_t M, N, splits, tokn, whole, tail, ldc, tiles_x, tiles_y, stages;
 
   // `whole` tiles, and those after them in `tail` pieces each
   __device__ __forceinline__ uint32_t total() const { return whole + (tiles_x * tiles_y * splits - whole) * tail; }
@@ -380,42 +377,43 @@ struct ProjectionWork {
   __device__ __forceinline__ void store(const Job &j, uint32_t row, uint32_t c, uint32_t (&r)[16]) const {
     const uint32_t n = j.w_row + row, t0 = j.x_row + c;
     if (t0 >= M) return;  // warp-uniform
-    if (OUT == kPairPartials) {
+    if (OUT == kGemmPartials) {
       if (n < N) {
 #pragma unroll
         for (uint32_t i = 0; i < 16; ++i)
           if (t0 + i < M) j.out[(size_t)(t0 + i) * ldc + n] = __uint_as_float(r[i]);
       }
-    } else if (OUT == kPairSwiglu || epilogue == kGemmGeglu) {
+    } else if (OUT == kGemmSwiglu || OUT == kGemmGeglu) {
       // Weight rows are interleaved: lane 2i holds gate f, lane 2i + 1 up f of these 16 tokens. The lanes of a pair trade halves and each
       // finishes one token of every two (SwiGLU: tensor.rs:167-189).
-      const uint32_t odd = row & 1u, stride = OUT == kPairSwiglu ? N >> 1 : ldc;
-      bf16 *out = act + (size_t)t0 * stride + (n >> 1);
+      const uint32_t odd = row & 1u;
+      const size_t stride = OUT == kGemmSwiglu ? N >> 1 : ldc;
+      bf16 *to = act + (t0 + odd) * stride + (n >> 1);
 #pragma unroll
-      for (uint32_t jj = 0; jj < 8; ++jj) {
-        const uint32_t recv = __shfl_xor_sync(0xffffffffu, odd ? r[2 * jj] : r[2 * jj + 1], 1), i = 2 * jj + odd;
+      for (uint32_t jj = 0; jj < 8; ++jj, to += 2 * stride) {
+        const uint32_t recv = __shfl_xor_sync(0xffffffffu, odd ? r[2 * jj] : r[2 * jj + 1], 1);
         const float g = __uint_as_float(odd ? recv : r[2 * jj]), u = __uint_as_float(odd ? r[2 * jj + 1] : recv);
-        const float v = OUT == kPairSwiglu ? __fmul_rn(g / (1.0f + __expf(-g)), u) : gelu_tanh<bf16>(g) * u;
-        if (t0 + i < M && n < N) out[(size_t)i * stride] = __float2bfloat16_rn(v);
+        const float v = OUT == kGemmSwiglu ? __fmul_rn(g / (1.0f + __expf(-g)), u) : gelu_tanh<bf16>(g) * u;
+        if (t0 + 2 * jj + odd < M && n < N) *to = __float2bfloat16_rn(v);
       }
     } else if (n < N) {
-      bf16 *out = act + (size_t)t0 * ldc + n;
+      bf16 *to = act + (size_t)t0 * ldc + n;
       const float b = bias ? bias[n] : 0.f;
 #pragma unroll
-      for (uint32_t i = 0; i < 16; ++i) {
+      for (uint32_t i = 0; i < 16; ++i, to += ldc) {
         const float v = __uint_as_float(r[i]) + b;
-        if (t0 + i < M) out[(size_t)i * ldc] = __float2bfloat16_rn(epilogue == kGemmGelu ? gelu_tanh<bf16>(v) : (epilogue == kGemmRelu2 ? relu2(v) : v));
+        if (t0 + i < M) *to = __float2bfloat16_rn(OUT == kGemmGelu ? gelu_tanh<bf16>(v) : (OUT == kGemmRelu2 ? relu2(v) : v));
       }
     }
   }
 };
 
-template <int OUT>
+template <GemmEpilogue OUT>
 __global__ void __launch_bounds__(PairConfig::kThreads)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_tail,
                  float *__restrict__ partial, bf16 *__restrict__ act, uint32_t M, uint32_t N, uint32_t K, uint32_t splits, uint32_t tokn, uint32_t whole,
-                 uint32_t tail, uint32_t ldc, uint32_t epilogue, ReadyWait ready, const float *__restrict__ bias) {
-  const ProjectionWork<OUT> work{&map_w, &map_x, &map_tail, partial, act, bias, M, N, splits, tokn, whole, tail, ldc, epilogue, (N + 2 * kTileN - 1) / (2 * kTileN),
+                 uint32_t tail, uint32_t ldc, ReadyWait ready, const float *__restrict__ bias) {
+  const ProjectionWork<OUT> work{&map_w, &map_x, &map_tail, partial, act, bias, M, N, splits, tokn, whole, tail, ldc, (N + 2 * kTileN - 1) / (2 * kTileN),
                                  (M + tokn - 1) / tokn, (K + PairConfig::kStageK - 1) / PairConfig::kStageK};
   run_pairs(work, ready, &g_gemm_error);
 }
@@ -525,11 +523,11 @@ uint32_t pair_splits(uint32_t rows, uint32_t n, uint32_t k) {
   return best;
 }
 
-template <int OUT>
+template <GemmEpilogue OUT>
 int launch_pair_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float *partial, bf16 *act, uint32_t rows, uint32_t n, uint32_t k,
-                     uint32_t splits, uint32_t ldc, GemmEpilogue epi, cudaStream_t stream, ReadyWait ready, const float *bias) {
+                     uint32_t splits, uint32_t ldc, cudaStream_t stream, ReadyWait ready, const float *bias) {
   if (ldc == 0) ldc = n;
-  if (ldc != n && (splits != 1 || epi == kGemmSwiglu))
+  if (ldc != n && (splits != 1 || OUT == kGemmSwiglu))
     return set_error(ORION_ERR_INTERNAL, "a strided GEMM output needs one k split and no SwiGLU");
   using Cfg = PairConfig;
   static bool attr_set[kMaxDeviceOrdinals] = {};
@@ -543,7 +541,7 @@ int launch_pair_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, f
   if (plan.tail > 1) ORION_TRY(cached_map(x, rows, k, ldx, tokn / plan.tail / 2, &mt));
   const uint32_t jobs = whole + (tiles - whole) * plan.tail;
   ORION_CUDA_CHECK("gemm_pair", launch_pdl_cluster(gemm_pair_kernel<OUT>, dim3(2 * std::min(jobs, kPairs)), dim3(Cfg::kThreads), dim3(2, 1, 1), Cfg::kSmemBytes,
-                                                   stream, mw, mx, mt, partial, act, rows, n, k, splits, tokn, whole, plan.tail, ldc, (uint32_t)epi, ready, bias));
+                                                   stream, mw, mx, mt, partial, act, rows, n, k, splits, tokn, whole, plan.tail, ldc, ready, bias));
   count_launch();
   ORION_CUDA_CHECK("gemm_pair", cudaGetLastError());
   return ORION_OK;
@@ -551,8 +549,13 @@ int launch_pair_form(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, f
 
 int launch_pair(const bf16 *x, uint32_t ldx, const bf16 *w, uint32_t ldw, float *partial, bf16 *act, uint32_t rows, uint32_t n, uint32_t k,
                 uint32_t splits, uint32_t ldc, GemmEpilogue epi, cudaStream_t stream, ReadyWait ready, const float *bias) {
-  auto form = epi == kGemmPartials ? launch_pair_form<kPairPartials> : (epi == kGemmSwiglu ? launch_pair_form<kPairSwiglu> : launch_pair_form<kPairAct>);
-  return form(x, ldx, w, ldw, partial, act, rows, n, k, splits, ldc, epi, stream, ready, bias);
+  auto form = epi == kGemmPartials ? launch_pair_form<kGemmPartials>
+              : epi == kGemmSwiglu ? launch_pair_form<kGemmSwiglu>
+              : epi == kGemmGelu   ? launch_pair_form<kGemmGelu>
+              : epi == kGemmRelu2  ? launch_pair_form<kGemmRelu2>
+              : epi == kGemmGeglu  ? launch_pair_form<kGemmGeglu>
+                                   : launch_pair_form<kGemmStore>;
+  return form(x, ldx, w, ldw, partial, act, rows, n, k, splits, ldc, stream, ready, bias);
 }
 
 // Who takes the persistent pairs: batches of more than 256 rows, with ORION_GEMM_PAIR=2 of more than 128 (the parity tests run this). The four

@@ -221,7 +221,6 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 // 2048 rows, experts of 2112 without gates, a shared one of 4224: 123 + 85 -> 88 + 70; 7006 rows, width 1024, 64 experts of 512: 150 + 94 -> 115 + 72.
 template <int GATED>
 struct MixtureWork {
-  static constexpr uint32_t kBatch = GATED ? 2 : 4;
   static constexpr bool kStaticTiles = false;
   struct Job : PairJob {
     MoeTile tile;
